@@ -39,37 +39,46 @@ __device__ __forceinline__ T jl_min(T x, T y) {
     return x < y ? x : y;
 }
 
+// The reduction and polynomial constants in constant memory: the multiply-adds read them as constant-bank operands,
+// so a step loop neither holds registers for them nor moves them into place.
+static __constant__ double c_red[5] = {CL_TWO_OVER_PI, CL_PIO2_1, CL_PIO2_2, CL_PIO2_3, 6755399441055744.0};
+static __constant__ double c_sin[8] = {CL_SIN_T17, CL_SIN_T15, CL_SIN_T13, CL_SIN_T11, CL_SIN_T9, CL_SIN_T7, CL_SIN_T5,
+                                       CL_SIN_T3};
+static __constant__ double c_cos[8] = {CL_COS_T16, CL_COS_T14, CL_COS_T12, CL_COS_T10, CL_COS_T8, CL_COS_T6, CL_COS_T4,
+                                       CL_COS_T2};
+
+// k = rint(p) and its quadrant k mod 4. For |p| < 2^51 the sum p + 1.5 2^52 rounds p to the integer (ties to even,
+// as rint), which its low word holds in two's complement: two additions instead of the conversions' ~30 cycles each.
+__device__ __forceinline__ double cl_quadrant(double p, int* q) {
+    const double t = p + c_red[4];
+    double k = t - c_red[4];
+    *q = __double2loint(t) & 3;
+    if (!(fabs(p) < 0x1p51)) {
+        k = rint(p);
+        *q = static_cast<int>(k - 4.0 * floor(k * 0.25));
+    }
+    return k;
+}
+
+// Both polynomials, then the quadrant by selects: 0 (s, c), 1 (c, -s), 2 (-s, -c), 3 (-c, s). A non-finite x reduces
+// to a NaN r and gives NaN; x = +-0 reduces to r = +0, so sin(x) = x is selected for the sign (tested on the bits).
 __device__ __forceinline__ void cl_sincos(double x, double* sn, double* cs) {
-    if (!isfin(x)) { *sn = x - x; *cs = x - x; return; }
-    if (x == 0.0) { *sn = x; *cs = 1.0; return; }
-    const double k = rint(x * CL_TWO_OVER_PI);
-    double r = fma(-k, CL_PIO2_1, x);
-    r = fma(-k, CL_PIO2_2, r);
-    r = fma(-k, CL_PIO2_3, r);
+    int q;
+    const double k = cl_quadrant(x * c_red[0], &q);
+    double r = fma(-k, c_red[1], x);
+    r = fma(-k, c_red[2], r);
+    r = fma(-k, c_red[3], r);
     const double z = r * r;
-    double ps = CL_SIN_T17;
-    ps = fma(ps, z, CL_SIN_T15);
-    ps = fma(ps, z, CL_SIN_T13);
-    ps = fma(ps, z, CL_SIN_T11);
-    ps = fma(ps, z, CL_SIN_T9);
-    ps = fma(ps, z, CL_SIN_T7);
-    ps = fma(ps, z, CL_SIN_T5);
-    ps = fma(ps, z, CL_SIN_T3);
-    const double s = fma(r * z, ps, r);
-    double pc = CL_COS_T16;
-    pc = fma(pc, z, CL_COS_T14);
-    pc = fma(pc, z, CL_COS_T12);
-    pc = fma(pc, z, CL_COS_T10);
-    pc = fma(pc, z, CL_COS_T8);
-    pc = fma(pc, z, CL_COS_T6);
-    pc = fma(pc, z, CL_COS_T4);
-    pc = fma(pc, z, CL_COS_T2);
-    const double c = fma(z, pc, 1.0);
-    const double q = k - 4.0 * floor(k * 0.25);
-    if (q == 0.0) { *sn = s; *cs = c; }
-    else if (q == 1.0) { *sn = c; *cs = -s; }
-    else if (q == 2.0) { *sn = -s; *cs = -c; }
-    else { *sn = -c; *cs = s; }
+    double ps = c_sin[0], pc = c_cos[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) { ps = fma(ps, z, c_sin[i]); pc = fma(pc, z, c_cos[i]); }
+    const double s = fma(r * z, ps, r), c = fma(z, pc, 1.0);
+    const bool odd = (q & 1) != 0;
+    const double a = odd ? c : s, b = odd ? s : c;
+    const long long fs = static_cast<long long>(q & 2) << 62, fc = static_cast<long long>((q + 1) & 2) << 62;
+    const double sv = __longlong_as_double(__double_as_longlong(a) ^ fs);
+    *sn = (__double_as_longlong(x) << 1) == 0 ? x : sv;
+    *cs = __longlong_as_double(__double_as_longlong(b) ^ fc);
 }
 // ---- split evaluation for the mixed kernels ------------------------------------------------------------------------
 // The same reduction as cl_sincos, then only the polynomial one Float64 value needs (the quadrant picks sin- or

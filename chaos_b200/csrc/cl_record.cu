@@ -68,7 +68,8 @@ struct RecOrbit {
             n += tau;
             const int8_t c = all_finite_x<D, S>(x) ? (all_finite<D * K>(W) ? STATUS_OK : STATUS_W) : STATUS_STATE;
             if (c != STATUS_OK) return c;
-            Est::template step<D, K>(est, n, W, prm);
+            int pend = 0;
+            Est::template step<D, K>(est, n, W, prm, pend);
             monitor_step(sys, x, mon);
             if (Est::template failed<D, K>(est)) return STATUS_REDUCER;
         }
