@@ -82,8 +82,7 @@ __device__ __forceinline__ void displaced(const double* x, const double* delta, 
 template <class Sys>
 __device__ __forceinline__ void fwd(const Sys& sys, double* z) {
     if constexpr (std::is_same<Sys, SysSplitHH>::value) {
-        SplitJac unused;
-        sys.forward(z, unused);
+        sys.step(z);
     } else {
         typename Sys::Jac J;
         sys.jac(z, J);
