@@ -8,9 +8,9 @@
 // (standard_map_chain.jl:38-60, chain_tangent.jl:53-91): each lane evaluates its own site's sine / cosine and its
 // right bond's, and takes the left bond's values and its neighbours' frame rows from the neighbouring lanes by warp
 // shuffles. At a handoff the group stages the frame in shared memory and runs QRSpectrum(HouseholderQR)
-// (householder.jl:19-80, qr_spectrum.jl:36-74) column-parallel: lane j owns columns j, j + G, ...; the owner of
-// column c builds reflector c in shared memory, every lane applies it to its own columns and forms its own columns
-// of Q. window_Gw (one lane) and orth_loss read R and Q from shared memory.
+// (householder.jl:19-80, qr_spectrum.jl:36-74) column-parallel (cl_coop_qr.cuh): lane j owns columns j, j + G, ...; the
+// owner of column c builds reflector c in shared memory, every lane applies it to its own columns and forms its own
+// columns of Q, then its columns of R^{-1} for window_Gw.
 //
 // Every entry is computed by the same operations, in the same order and type, as in the one-thread kernel: the
 // band product's sums, every left-folded dot product and norm, the reflectors' zero rows. Only the lane doing the
@@ -18,63 +18,19 @@
 // Maxima combined across lanes (orth_loss, the escape test) use operations whose result does not depend on order.
 #pragma once
 
+#include "cl_coop_qr.cuh"
 #include "cl_ensemble.cuh"
 
 namespace cl {
 
 // Shared-memory words of one orbit's handoff workspace (in Real): the staged frame (D x K), Q (D x K), the
-// reflectors (D x NREF; afterwards window_Gw's scratch column) and R (K x K).
+// reflectors (D x NREF; afterwards R^{-1}'s triangle) and R (K x K).
 template <int D, int K>
 struct CoopSmem {
-    static constexpr int NREF = K < D ? K : K - 1;
-    static constexpr int T = D * K, Q = D * K, U = (D * NREF > K ? D * NREF : K), R = K * K;
+    static constexpr int NREF = K < D ? K : K - 1, TRI = K * (K + 1) / 2;
+    static constexpr int T = D * K, Q = D * K, U = (D * NREF > TRI ? D * NREF : TRI), R = K * K;
     static constexpr int words = T + Q + U + R;
 };
-
-template <int G>
-__device__ __forceinline__ unsigned group_mask(int lane) {
-    return G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
-}
-
-template <int G>
-__device__ __forceinline__ bool group_all(unsigned mask, bool p) {
-    return (__ballot_sync(mask, p) & mask) == mask;
-}
-
-template <typename T>
-__device__ __forceinline__ T rv(const T* R0, int l, bool rescale, T m) { return rescale ? dv(R0[l], m) : R0[l]; }
-
-// window_Gw (orthonormalize.jl:112-127) on R in shared memory, one column of R^{-1} at a time (scratch `ri`, K
-// words): the same operations in the same order as the register version in cl_qr.cuh. The two Frobenius sums are
-// independent left folds in column-major order, so folding the inverse column by column changes nothing.
-template <int K, typename T>
-__device__ __forceinline__ T window_Gw_sm(const T* R0, T* ri) {
-    T m = fabs(R0[0]);
-#pragma unroll 1
-    for (int l = 1; l < K * K; ++l) m = mx(m, static_cast<T>(fabs(R0[l])));
-    bool rescale = false;
-    if constexpr (sizeof(T) == 8) rescale = (m > T(1e100) || m < T(1e-100)) && isfin(m) && m > T(0);
-    T a = rv(R0, 0, rescale, m) * rv(R0, 0, rescale, m);
-#pragma unroll 1
-    for (int l = 1; l < K * K; ++l) a = a + rv(R0, l, rescale, m) * rv(R0, l, rescale, m);
-    T b = T(0);
-#pragma unroll 1
-    for (int jc = 0; jc < K; ++jc) {
-#pragma unroll 1
-        for (int i = 0; i < K; ++i) ri[i] = T(0);
-        ri[jc] = dv(T(1), rv(R0, jc + jc * K, rescale, m));
-#pragma unroll 1
-        for (int i = jc - 1; i >= 0; --i) {
-            T s = T(0);
-#pragma unroll 1
-            for (int l = i + 1; l <= jc; ++l) s = s + rv(R0, i + l * K, rescale, m) * ri[l];
-            ri[i] = dv(-s, rv(R0, i + i * K, rescale, m));
-        }
-#pragma unroll 1
-        for (int i = 0; i < K; ++i) b = (jc == 0 && i == 0) ? ri[0] * ri[0] : b + ri[i] * ri[i];
-    }
-    return sqt(a) * sqt(b);
-}
 
 // One lane's part of QRState<K>: the sums of its own columns; the scalars are kept identical in every lane.
 template <int K, int KPL>
@@ -219,104 +175,8 @@ __global__ void __launch_bounds__(128, MINB) coop_kernel(const EArgs a, const Sy
                 for (int m = 0; m < KPL; ++m)
 #pragma unroll
                     for (int r = 0; r < D; ++r) A[m][r] = sT[(j + m * G) * D + r];
-                // _hh_sweep (householder.jl:19-50): reflector jj is built in place in shared memory by the owner of
-                // column jj (zero when the column's norm is zero or not finite) and applied by every lane
-                int count = 0;
-#pragma unroll
-                for (int jj = 0; jj < NREF; ++jj) {
-                    const int owner = jj % G, mj = jj / G;
-                    Real* u = sU + jj * D;
-                    int okv = 0;
-                    Real rho = Real(0);
-                    if (j == owner) {
-#pragma unroll
-                        for (int m = 0; m < KPL; ++m)   // A[mj] with compile-time indices (jj need not unroll)
-                            if (m == mj) {
-#pragma unroll
-                                for (int r = 0; r < D; ++r) u[r] = r >= jj ? A[m][r] : Real(0);
-                            }
-                        const Real cn = nrm<D>(u);
-                        if (isfin(cn) && cn > Real(0)) {
-                            const Real sg = u[jj] < Real(0) ? Real(-1) : Real(1);
-                            u[jj] = u[jj] + sg * cn;
-                            const Real nv = nrm<D>(u);
-#pragma unroll
-                            for (int r = 0; r < D; ++r) u[r] = dv(u[r], nv);
-                            rho = -sg * cn;
-                            okv = 1;
-                        } else {
-#pragma unroll
-                            for (int r = 0; r < D; ++r) u[r] = Real(0);
-                            rho = cn;
-                        }
-                    }
-                    __syncwarp(gm);
-                    if (__shfl_sync(gm, okv, owner, G)) {
-#pragma unroll
-                        for (int m = 0; m < KPL; ++m) {
-                            const Real w = dotv<D>(u, A[m]);
-#pragma unroll
-                            for (int r = 0; r < D; ++r) A[m][r] = A[m][r] - (Real(2) * u[r]) * w;
-                        }
-                        count += 1;
-                    }
-                    if (j == owner) {
-#pragma unroll
-                        for (int m = 0; m < KPL; ++m)
-#pragma unroll
-                            for (int r = 0; r < D; ++r)
-                                if (m == mj && r == jj) A[m][r] = rho;
-                    }
-                }
-                // _finish (householder.jl:66-75): R's rows of this lane's columns, the signs of the diagonal (a bit
-                // mask, read by every lane before any column is rewritten), then the sign-fixed upper triangle
-#pragma unroll
-                for (int m = 0; m < KPL; ++m)
-#pragma unroll
-                    for (int r = 0; r < K; ++r) sR[r + (j + m * G) * K] = A[m][r];
-                __syncwarp(gm);
-                unsigned neg = 0;
-#pragma unroll
-                for (int r = 0; r < K; ++r) neg |= (sR[r + r * K] < Real(0) ? 1u : 0u) << r;
-                __syncwarp(gm);
-#pragma unroll
-                for (int m = 0; m < KPL; ++m) {
-                    const int cc = j + m * G;
-#pragma unroll
-                    for (int r = 0; r < K; ++r) {
-                        const Real sgr = (neg >> r) & 1u ? Real(-1) : Real(1);
-                        sR[r + cc * K] = r > cc ? Real(0) : sgr * sR[r + cc * K];
-                    }
-                }
-                // Q = the reflectors applied to I[:, 1:K] in reverse (householder.jl:77-80), then the signs
-#pragma unroll
-                for (int m = 0; m < KPL; ++m)
-#pragma unroll
-                    for (int r = 0; r < D; ++r) A[m][r] = r == j + m * G ? Real(1) : Real(0);
-#pragma unroll
-                for (int jj = NREF - 1; jj >= 0; --jj) {
-                    const Real* u = sU + jj * D;
-#pragma unroll
-                    for (int m = 0; m < KPL; ++m) {
-                        const Real w = dotv<D>(u, A[m]);
-#pragma unroll
-                        for (int r = 0; r < D; ++r) A[m][r] = A[m][r] - (Real(2) * u[r]) * w;
-                    }
-                }
-#pragma unroll
-                for (int m = 0; m < KPL; ++m) {
-                    const int cc = j + m * G;
-                    const Real sgc = (neg >> cc) & 1u ? Real(-1) : Real(1);
-#pragma unroll
-                    for (int r = 0; r < D; ++r) { A[m][r] = A[m][r] * sgc; sQ[cc * D + r] = A[m][r]; }
-                }
-                __syncwarp(gm);
-                int status = QR_OK, fcol = 0;
-#pragma unroll
-                for (int jj = K - 1; jj >= 0; --jj) {
-                    const Real pv = sR[jj + jj * K];
-                    if (!(isfin(pv) && pv > Real(0))) { status = QR_PIVOT; fcol = jj + 1; }
-                }
+                const CoopFactor f = coop_householder<D, K, G>(A, sQ, sU, sR, gm, j);
+                const int status = f.status, fcol = f.column, count = f.count;
                 // QRSpectrum's step (qr_spectrum.jl:36-74)
                 bool replace = false;
                 if (status != QR_OK) {
@@ -328,30 +188,8 @@ __global__ void __launch_bounds__(128, MINB) coop_kernel(const EArgs a, const Sy
                     st.step = n;
                 } else {
                     const Real epsT = Eps<Real>::eps();
-                    Real Gw = Real(0);
-                    if (j == 0) Gw = window_Gw_sm<K>(sR, sU);   // the reflectors are spent: sU is scratch
-                    Gw = __shfl_sync(gm, Gw, 0, G);
-                    // orth_loss: this lane's columns of the upper triangle of Q'Q, then the maximum over the group
-                    Real om = Real(0);
-                    bool first = true;
-#pragma unroll
-                    for (int m = 0; m < KPL; ++m) {
-                        const int cc = j + m * G;
-#pragma unroll
-                        for (int r = 0; r < K; ++r) {
-                            if (r > cc) continue;
-                            const Real* qi = sQ + r * D;
-                            Real acc = qi[0] * A[m][0];
-#pragma unroll
-                            for (int l = 1; l < D; ++l) acc = fma(qi[l], A[m][l], acc);
-                            if (r == cc) acc = acc - Real(1);
-                            const Real av = fabs(acc);
-                            om = first ? av : mx(om, av);
-                            first = false;
-                        }
-                    }
-#pragma unroll
-                    for (int off = G / 2; off >= 1; off >>= 1) om = mx(om, __shfl_xor_sync(gm, om, off, G));
+                    const Real Gw = coop_window_Gw<K, G>(sR, sU, gm, j);   // the reflectors are spent: sU is scratch
+                    const Real om = coop_orth<D, K, G>(A, sQ, gm, j);
                     const Real orth = K >= 2 ? om : Real(0);
                     const Real thr = static_cast<Real>(a.prm[0].orthogonality_tol) * epsT * static_cast<Real>(K);
                     if (K >= 2 && !(orth <= thr)) {
@@ -359,7 +197,7 @@ __global__ void __launch_bounds__(128, MINB) coop_kernel(const EArgs a, const Sy
                         st.threshold = static_cast<double>(thr); st.step = n;
                     } else {
 #pragma unroll
-                        for (int m = 0; m < KPL; ++m) cs_add(st.sums[m], lnr(sR[(j + m * G) * (K + 1)]));
+                        for (int m = 0; m < KPL; ++m) cs_add(st.sums[m], coop_log(sR[(j + m * G) * (K + 1)]));
                         const Real Gq = G_from_Gw<K>(Gw);
                         st.n = n;
                         st.G_max = jl_max(st.G_max, static_cast<double>(Gq));

@@ -27,8 +27,7 @@ template <int NS> struct CoopWidth { static constexpr int G = NS <= 2 ? 2 : NS <
 // QRSpectrum on the staged frame, column-parallel (qr_spectrum.jl:36-74): lane j owns columns j, j + G, ... The
 // QRState sums of this lane's columns and the shared scalars (kept equal in every lane) are read from and written
 // back to the Julia-layout state `st` in shared memory by lane 0 / the column owners. Returns true on failure.
-//   HouseholderQR (householder.jl:19-80): the owner of column jj builds reflector jj in shared memory, every lane
-//   applies it to its own columns and forms its own columns of Q.
+//   HouseholderQR (householder.jl:19-80): coop_householder (cl_coop_qr.cuh).
 //   MGS (orthonormalize.jl:49-58, 88-105): in round r the owner of column r, projected already on q_0 .. q_{r-1},
 //   takes its norm and normalises it into q_r (the first column whose norm fails stops the factorisation, as the
 //   serial loop does); then every lane projects its later columns on q_r (c = q_r . u, u - c q_r): each column sees
@@ -36,7 +35,6 @@ template <int NS> struct CoopWidth { static constexpr int G = NS <= 2 ? 2 : NS <
 template <int ALG, int D, int K, int G, typename Real>
 __device__ __forceinline__ bool coop_qr_step(QRState<K>& st, i64 n, Real* sT, Real* sQ, Real* sU, Real* sR,
                                              unsigned gm, int j, double orth_tol) {
-    constexpr int NREF = K < D ? K : K - 1;
     constexpr int KPL = (K + G - 1) / G;   // columns per lane (the last lanes may own fewer)
     constexpr bool HH = ALG == CL_QR_HOUSEHOLDER;
     Real A[KPL][D];
@@ -62,14 +60,15 @@ __device__ __forceinline__ bool coop_qr_step(QRState<K>& st, i64 n, Real* sT, Re
 #pragma unroll
                 for (int m = 0; m < KPL; ++m) {
                     if (m != mo) continue;
-                    const Real gamma = nrm<D>(A[m]);
+                    const Real gamma = coop_norm<D>(A[m]);
 #pragma unroll
                     for (int i = 0; i < K; ++i) sR[i + rr * K] = i < rr ? Rc[m][i] : (i == rr ? gamma : Real(0));
                     if (!(isfin(gamma) && gamma > Real(0))) {
                         bad = 1;
                     } else {
+                        coop_divide<D>(A[m], gamma, A[m]);
 #pragma unroll
-                        for (int l = 0; l < D; ++l) { A[m][l] = dv(A[m][l], gamma); sQ[rr * D + l] = A[m][l]; }
+                        for (int l = 0; l < D; ++l) sQ[rr * D + l] = A[m][l];
                     }
                 }
             }
@@ -88,106 +87,11 @@ __device__ __forceinline__ bool coop_qr_step(QRState<K>& st, i64 n, Real* sT, Re
             __syncwarp(gm);
         }
     } else {
-#pragma unroll
-    for (int jj = 0; jj < NREF; ++jj) {
-        const int owner = jj % G, mj = jj / G;
-        Real* u = sU + jj * D;
-        int okv = 0;
-        Real rho = Real(0);
-        if (j == owner) {
-#pragma unroll
-            for (int m = 0; m < KPL; ++m)
-                if (m == mj) {
-#pragma unroll
-                    for (int r = 0; r < D; ++r) u[r] = r >= jj ? A[m][r] : Real(0);
-                }
-            const Real cn = nrm<D>(u);
-            if (isfin(cn) && cn > Real(0)) {
-                const Real sg = u[jj] < Real(0) ? Real(-1) : Real(1);
-                u[jj] = u[jj] + sg * cn;
-                const Real nv = nrm<D>(u);
-#pragma unroll
-                for (int r = 0; r < D; ++r) u[r] = dv(u[r], nv);
-                rho = -sg * cn;
-                okv = 1;
-            } else {
-#pragma unroll
-                for (int r = 0; r < D; ++r) u[r] = Real(0);
-                rho = cn;
-            }
-        }
-        __syncwarp(gm);
-        if (__shfl_sync(gm, okv, owner, G)) {
-#pragma unroll
-            for (int m = 0; m < KPL; ++m) {
-                if (j + m * G >= K) continue;
-                const Real w = dotv<D>(u, A[m]);
-#pragma unroll
-                for (int r = 0; r < D; ++r) A[m][r] = A[m][r] - (Real(2) * u[r]) * w;
-            }
-            count += 1;
-        }
-        if (j == owner) {
-#pragma unroll
-            for (int m = 0; m < KPL; ++m)
-#pragma unroll
-                for (int r = 0; r < D; ++r)
-                    if (m == mj && r == jj) A[m][r] = rho;
-        }
+        const CoopFactor f = coop_householder<D, K, G>(A, sQ, sU, sR, gm, j);
+        count = f.count;
+        status = f.status;
+        fcol = f.column;
     }
-    // _finish (householder.jl:66-75)
-#pragma unroll
-    for (int m = 0; m < KPL; ++m) {
-        const int cc = j + m * G;
-        if (cc >= K) continue;
-#pragma unroll
-        for (int r = 0; r < K; ++r) sR[r + cc * K] = A[m][r];
-    }
-    __syncwarp(gm);
-    unsigned neg = 0;
-#pragma unroll
-    for (int r = 0; r < K; ++r) neg |= (sR[r + r * K] < Real(0) ? 1u : 0u) << r;
-    __syncwarp(gm);
-#pragma unroll
-    for (int m = 0; m < KPL; ++m) {
-        const int cc = j + m * G;
-        if (cc >= K) continue;
-#pragma unroll
-        for (int r = 0; r < K; ++r) {
-            const Real sgr = (neg >> r) & 1u ? Real(-1) : Real(1);
-            sR[r + cc * K] = r > cc ? Real(0) : sgr * sR[r + cc * K];
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < KPL; ++m)
-#pragma unroll
-        for (int r = 0; r < D; ++r) A[m][r] = r == j + m * G ? Real(1) : Real(0);
-#pragma unroll
-    for (int jj = NREF - 1; jj >= 0; --jj) {
-        const Real* u = sU + jj * D;
-#pragma unroll
-        for (int m = 0; m < KPL; ++m) {
-            if (j + m * G >= K) continue;
-            const Real w = dotv<D>(u, A[m]);
-#pragma unroll
-            for (int r = 0; r < D; ++r) A[m][r] = A[m][r] - (Real(2) * u[r]) * w;
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < KPL; ++m) {
-        const int cc = j + m * G;
-        if (cc >= K) continue;
-        const Real sgc = (neg >> cc) & 1u ? Real(-1) : Real(1);
-#pragma unroll
-        for (int r = 0; r < D; ++r) { A[m][r] = A[m][r] * sgc; sQ[cc * D + r] = A[m][r]; }
-    }
-    __syncwarp(gm);
-#pragma unroll
-    for (int jj = K - 1; jj >= 0; --jj) {
-        const Real pv = sR[jj + jj * K];
-        if (!(isfin(pv) && pv > Real(0))) { status = QR_PIVOT; fcol = jj + 1; }
-    }
-    }   // HouseholderQR
     bool replace = false, fail = false;
     if (status != QR_OK) {
         Real pv = sR[0];
@@ -201,9 +105,7 @@ __device__ __forceinline__ bool coop_qr_step(QRState<K>& st, i64 n, Real* sT, Re
         fail = true;
     } else {
         const Real epsT = Eps<Real>::eps();
-        Real Gw = Real(0);
-        if (j == 0) Gw = window_Gw_sm<K>(sR, sU);   // the reflectors are spent: sU is scratch
-        Gw = __shfl_sync(gm, Gw, 0, G);
+        const Real Gw = coop_window_Gw<K, G>(sR, sU, gm, j);   // the reflectors are spent: sU is scratch
         // conditioning (the Gram-Schmidt family only, qr_spectrum.jl:54-58)
         if (!HH && !(static_cast<double>(Gw * epsT) < 0.5)) {
             if (j == 0) {
@@ -212,29 +114,7 @@ __device__ __forceinline__ bool coop_qr_step(QRState<K>& st, i64 n, Real* sT, Re
             __syncwarp(gm);
             return true;
         }
-        Real om = Real(0);
-        bool first = true;
-#pragma unroll
-        for (int m = 0; m < KPL; ++m) {
-            const int cc = j + m * G;
-            if (cc >= K) continue;
-#pragma unroll
-            for (int r = 0; r < K; ++r) {
-                if (r > cc) continue;
-                const Real* qi = sQ + r * D;
-                Real acc = qi[0] * A[m][0];
-#pragma unroll
-                for (int l = 1; l < D; ++l) acc = fma(qi[l], A[m][l], acc);
-                if (r == cc) acc = acc - Real(1);
-                const Real av = fabs(acc);
-                om = first ? av : mx(om, av);
-                first = false;
-            }
-        }
-        // the maximum over the group: every lane owns at least one column (K >= G), and the NaN-aware maximum of
-        // non-negative values does not depend on the order it combines them in
-#pragma unroll
-        for (int off = G / 2; off >= 1; off >>= 1) om = mx(om, __shfl_xor_sync(gm, om, off, G));
+        const Real om = coop_orth<D, K, G>(A, sQ, gm, j);
         const Real orth = K >= 2 ? om : Real(0);
         const Real thr = static_cast<Real>(orth_tol) * epsT * static_cast<Real>(K) * (HH ? Real(1) : Gw);
         if (K >= 2 && !(orth <= thr)) {
@@ -247,7 +127,7 @@ __device__ __forceinline__ bool coop_qr_step(QRState<K>& st, i64 n, Real* sT, Re
 #pragma unroll
             for (int m = 0; m < KPL; ++m) {
                 const int cc = j + m * G;
-                if (cc < K) cs_add(st.sums[cc], lnr(sR[cc * (K + 1)]));
+                if (cc < K) cs_add(st.sums[cc], coop_log(sR[cc * (K + 1)]));
             }
             if (j == 0) {
                 const Real Gq = G_from_Gw<K>(Gw);
@@ -276,11 +156,9 @@ __device__ __forceinline__ bool coop_qr_step(QRState<K>& st, i64 n, Real* sT, Re
 
 // GALI (gali.jl:17-201, the frame's unit columns and _gram_core! at :81-100) on the staged frame, column-parallel:
 // every lane takes its own columns' norms, log sums and unit columns; the first failing column over the group (the
-// lowest index) stops the step as the serial loop does. The twice-orthogonalised Gram core runs by rounds: in round r
-// the owner of column r, projected already once on the final q_0 .. q_{r-1}, projects it a second time on all of them,
-// takes its norm and normalises it, and G_r = G_{r-1} r_r is formed in every lane from the broadcast norm; then every
-// lane makes the first projection of its later columns on q_r. Each column sees the serial loop's projections in its
-// order. The frame becomes the unit columns (not Q). Returns true on failure.
+// lowest index) stops the step as the serial loop does. The frame becomes the unit columns, kept in sQ as well: the
+// values G_2..G_k are a function of them that every later successful handoff overwrites, so they are formed once, from
+// the last ones (coop_gali_values). Returns true on failure.
 template <int D, int K, int G, typename Real>
 __device__ __forceinline__ bool coop_gali_step(GALIState<K>& st, i64 n, Real* sT, Real* sQ, unsigned gm, int j) {
     constexpr int KPL = (K + G - 1) / G;
@@ -292,7 +170,7 @@ __device__ __forceinline__ bool coop_gali_step(GALIState<K>& st, i64 n, Real* sT
         if (cc >= K) continue;
 #pragma unroll
         for (int r = 0; r < D; ++r) A[m][r] = sT[cc * D + r];
-        a[m] = nrm<D>(A[m]);
+        a[m] = coop_norm<D>(A[m]);
         if (!(isfin(a[m]) && a[m] >= Eps<Real>::floatmin())) mybad = cc + 1;
     }
     const int bad = __reduce_min_sync(gm, static_cast<unsigned>(mybad));
@@ -311,11 +189,32 @@ __device__ __forceinline__ bool coop_gali_step(GALIState<K>& st, i64 n, Real* sT
         const int cc = j + m * G;
         if (cc >= K) continue;
         CS acc{st.s[cc], st.c[cc]};
-        cs_add(acc, lnr(a[m]));
+        cs_add(acc, coop_log(a[m]));
         st.s[cc] = acc.s; st.c[cc] = acc.c;
+        coop_divide<D>(A[m], a[m], A[m]);
 #pragma unroll
-        for (int r = 0; r < D; ++r) { A[m][r] = dv(A[m][r], a[m]); sT[cc * D + r] = A[m][r]; }
+        for (int r = 0; r < D; ++r) { sT[cc * D + r] = A[m][r]; sQ[cc * D + r] = A[m][r]; }
     }
+    if (j == 0) st.n = n;
+    __syncwarp(gm);
+    return false;
+}
+
+// G_2..G_k (_gram_core!, gali.jl:81-100) of the unit columns in sQ, by rounds: in round r the owner of column r,
+// projected already once on the final q_0 .. q_{r-1}, projects it a second time on all of them, takes its norm and
+// normalises it, and G_r = G_{r-1} r_r is formed in every lane from the broadcast norm; then every lane makes the first
+// projection of its later columns on q_r. Each column sees the serial loop's projections in its order.
+template <int D, int K, int G, typename Real>
+__device__ __forceinline__ void coop_gali_values(GALIState<K>& st, Real* sQ, unsigned gm, int j) {
+    constexpr int KPL = (K + G - 1) / G;
+    Real A[KPL][D];
+#pragma unroll
+    for (int m = 0; m < KPL; ++m) {
+        const int cc = j + m * G;
+#pragma unroll
+        for (int r = 0; r < D; ++r) A[m][r] = cc < K ? sQ[cc * D + r] : Real(0);
+    }
+    __syncwarp(gm);
     Real g = Real(1);
 #pragma unroll
     for (int rr = 0; rr < K; ++rr) {
@@ -334,10 +233,10 @@ __device__ __forceinline__ bool coop_gali_step(GALIState<K>& st, i64 n, Real* sT
 #pragma unroll
                     for (int i = 0; i < D; ++i) A[m][i] = A[m][i] - cc * qp[i];
                 }
-                rn = nrm<D>(A[m]);
-                const Real sc = rn == Real(0) ? Real(1) : rn;
+                rn = coop_norm<D>(A[m]);
+                coop_divide<D>(A[m], rn == Real(0) ? Real(1) : rn, A[m]);
 #pragma unroll
-                for (int i = 0; i < D; ++i) { A[m][i] = dv(A[m][i], sc); sQ[rr * D + i] = A[m][i]; }
+                for (int i = 0; i < D; ++i) sQ[rr * D + i] = A[m][i];
             }
         }
         rn = __shfl_sync(gm, rn, owner, G);
@@ -358,9 +257,7 @@ __device__ __forceinline__ bool coop_gali_step(GALIState<K>& st, i64 n, Real* sT
             for (int i = 0; i < D; ++i) A[m][i] = A[m][i] - c * qr_[i];
         }
     }
-    if (j == 0) st.n = n;
     __syncwarp(gm);
-    return false;
 }
 
 // The column-parallel QR runs when every lane owns at least one column (K >= G): HouseholderQR in both precisions,
@@ -384,9 +281,9 @@ __global__ void __launch_bounds__(128) coop_orbit_kernel(const KArgs a, const Sy
     using Ch = typename F0::template Chain_<D>;
     constexpr int words = Ch::bytes / 8;
     constexpr bool HH = CoopQRForm<F0, Real, G>::value || CoopGaliForm<F0, Real, G>::value;   // shared-memory workspace
-    constexpr int NREF = K < D ? K : K - 1;
+    constexpr int NREF = K < D ? K : K - 1, TRI = K * (K + 1) / 2;
     // per group: the staged frame, then (Householder) Q, the reflectors and R, then the chain's state
-    constexpr int FW = D * K, QW = HH ? D * K : 0, UW = HH ? (D * NREF > K ? D * NREF : K) : 0, RW = HH ? K * K : 0;
+    constexpr int FW = D * K, QW = HH ? D * K : 0, UW = HH ? (D * NREF > TRI ? D * NREF : TRI) : 0, RW = HH ? K * K : 0;
     constexpr int REAL_WORDS = FW + QW + UW + RW;
     constexpr int GROUP_BYTES = ((REAL_WORDS * static_cast<int>(sizeof(Real)) + 7) / 8) * 8 + words * 8;
     static_assert(32 % G == 0 && G >= NS, "group shape");
@@ -442,7 +339,7 @@ __global__ void __launch_bounds__(128) coop_orbit_kernel(const KArgs a, const Sy
     __syncwarp(gm);
 
     i64 n = a.n0;
-    bool alive = true;
+    bool alive = true, pending = false;   // pending: GALI's values are still to be formed
     const i64 handoffs = a.steps / a.tau;
     for (i64 h = 0; h < handoffs; ++h) {
         for (int t = 0; t < a.tau; ++t) L.step(gm, jl, jr, hasL, hasR, sys.K, sys.eps);
@@ -467,6 +364,7 @@ __global__ void __launch_bounds__(128) coop_orbit_kernel(const KArgs a, const Sy
             } else if constexpr (CoopGaliForm<F0, Real, G>::value) {
                 GALIState<K>& st = *reinterpret_cast<GALIState<K>*>(sSt);
                 failed = coop_gali_step<D, K, G>(st, n, sT, sQ, gm, j) ? 1 : 0;
+                if (!failed) pending = true;
             } else {
                 if (j == 0) {
                     Ch ch;
@@ -486,6 +384,9 @@ __global__ void __launch_bounds__(128) coop_orbit_kernel(const KArgs a, const Sy
             if (failed) c0 = STATUS_REDUCER;
         }
         if (c0 != STATUS_OK) { code = c0; hstep = n; alive = false; break; }
+    }
+    if constexpr (CoopGaliForm<F0, Real, G>::value) {
+        if (pending) coop_gali_values<D, K, G>(*reinterpret_cast<GALIState<K>*>(sSt), sQ, gm, j);
     }
     if (alive) {   // orbit.jl:58: the final status check runs only at step N
         bool fw = true;
@@ -517,8 +418,8 @@ template <int NS, typename Real, class F0>
 cudaError_t launch_coop_orbit(const cl_run& run, const KArgs& a, cudaStream_t st, LaunchInfo* info) {
     constexpr int G = CoopWidth<NS>::G, D = 2 * NS, K = F0::K;
     constexpr bool HH = CoopQRForm<F0, Real, G>::value || CoopGaliForm<F0, Real, G>::value;   // shared-memory workspace
-    constexpr int NREF = K < D ? K : K - 1;
-    constexpr int FW = D * K, QW = HH ? D * K : 0, UW = HH ? (D * NREF > K ? D * NREF : K) : 0, RW = HH ? K * K : 0;
+    constexpr int NREF = K < D ? K : K - 1, TRI = K * (K + 1) / 2;
+    constexpr int FW = D * K, QW = HH ? D * K : 0, UW = HH ? (D * NREF > TRI ? D * NREF : TRI) : 0, RW = HH ? K * K : 0;
     constexpr int words = F0::template Chain_<D>::bytes / 8;
     constexpr int GROUP_BYTES = (((FW + QW + UW + RW) * static_cast<int>(sizeof(Real)) + 7) / 8) * 8 + words * 8;
     const SysChain<NS> sys = SysMaker<SysChain<NS>>::make(run, nullptr);

@@ -109,9 +109,15 @@ __device__ __forceinline__ double log64(double x) {
 // Only the first n <= N entries count (n a constant of the caller's unrolled loop).
 template <int N>
 __device__ __forceinline__ double norm64(const double* v, Ok& ok, int n = N) {
-    double m = fabs(v[0]);
+    double t[N];
 #pragma unroll
-    for (int i = 1; i < N; ++i) if (i < n) { const double a = fabs(v[i]); m = a > m ? a : m; }
+    for (int i = 0; i < N; ++i) t[i] = i < n ? fabs(v[i]) : 0.0;
+#pragma unroll
+    for (int w = 8; w >= 1; w >>= 1)   // the maximum as a tree (a compare and select cost 19 cycles of latency)
+#pragma unroll
+        for (int i = 0; i < N && i < w; ++i)
+            if (i + w < N && i + w < n) t[i] = t[i + w] > t[i] ? t[i + w] : t[i];
+    const double m = t[0];
     ok.positive<700>(m);
     const double y = rcp64(m);
     double q = quo64z(v[0], m, y);

@@ -9,6 +9,7 @@
 // the results are bit-identical to the CPU oracle's restatement.
 #pragma once
 
+#include "../../include/chaoslab_b200.h"
 #include "cl_math.cuh"
 
 namespace cl {
