@@ -121,6 +121,10 @@ struct SysPair {
 template <class Sys> __device__ __forceinline__ const Sys& monitored(const Sys& s) { return s; }
 template <class Base> __device__ __forceinline__ const Base& monitored(const SysPair<Base>& s) { return s.base; }
 
+template <class J> __device__ __forceinline__ auto monitored_jac(const J& j) -> decltype((j.A)) { return j.A; }
+__device__ __forceinline__ const StdJac& monitored_jac(const StdJac& j) { return j; }
+__device__ __forceinline__ const SysLinear<2>::Jac& monitored_jac(const SysLinear<2>::Jac& j) { return j; }
+
 // _put_members! over the compile-time chain
 template <int D, int K>
 __device__ __forceinline__ int put_members(const Chain<D, K>&, double*) { return 0; }
@@ -139,19 +143,25 @@ struct IndOrbit {
     double x[S], W[D * K];
     Ch ch;
     MonState mon;
+    typename Sys::Jac J;   // the tangent entries at x, for the next step and the monitor (as the study recorder's)
     __device__ __forceinline__ int8_t body(const Sys& sys, i64& n, i64 steps, const IndArgs& a) {
         for (i64 hh = 0; hh < steps / a.tau; ++hh) {
-            for (int t = 0; t < a.tau; ++t) {
-                typename Sys::Jac J;
-                sys.jac(x, J);
+            for (int t = 1; t < a.tau; ++t) {
                 sys.template apply<K>(J, W);
                 sys.forward(x, J);
+                sys.jac(x, J);
             }
+            sys.template apply<K>(J, W);
+            sys.forward(x, J);
+            sys.jac(x, J);
+            typename F::template Measure_<D, double> m;
+            m.take(W, a.prm);
             n += a.tau;
             const int8_t cc = all_finite_x<D, S>(x) ? (all_finite<D * K>(W) ? STATUS_OK : STATUS_W) : STATUS_STATE;
             if (cc != STATUS_OK) return cc;
-            ch.step(n, W, a.prm);
-            monitor_step(monitored(sys), x, mon);
+            int pend = 0;
+            ch.template run<true, false>(n, W, a.prm, m, pend);
+            monitor_ahead(monitored(sys), x, monitored_jac(J), mon);
             if (ch.failed()) return STATUS_REDUCER;
         }
         return n == a.N ? (all_finite_x<D, S>(x) ? (all_finite<D * K>(W) ? STATUS_OK : STATUS_W) : STATUS_STATE)
@@ -183,6 +193,7 @@ __global__ void __launch_bounds__(128) ind_series_kernel(const IndArgs a, const 
 #pragma unroll
         for (int w = 0; w < MW; ++w) mw[w] = st[CW + w];
     }
+    sys.jac(o.x, o.J);
     i64 n = a.n0, h = a.n0;
     int8_t c = STATUS_OK;
     int glo = 0;

@@ -27,33 +27,44 @@ __device__ __forceinline__ void dense_tangent(const Sys& sys, const double* x, d
     }
 }
 
-// RunMonitor's step (run_record.jl:37-40): det of a 2 x 2 static matrix M[1] M[4] - M[3] M[2]; M' Omega M by the
-// StaticArrays products (the fused chain); Julia's NaN-propagating max.
+// Julia's max of two non-negative values, without a branch: NaN if either is NaN (two zeros are both +0)
+__device__ __forceinline__ double max_nonneg(double x, double y) { return x >= y || x != x ? x : y; }
+
+// RunMonitor's step (run_record.jl:37-40) on the tangent M: det of a 2 x 2 static matrix M[1] M[4] - M[3] M[2]; M' Omega
+// M by the StaticArrays products (the fused chain; Omega's zeros and ones leave M' Omega = [-M[2] M[1]; -M[4] M[3]] for a
+// finite M, and the point is finite here); Julia's NaN-propagating max.
+__device__ __forceinline__ void monitor_tangent(const double* M, MonState& m) {
+    const double edet = fabs((M[0] * M[3] - M[2] * M[1]) - 1.0);
+    const double P[4] = {-M[1], -M[3], M[0], M[2]};
+    const double Om[4] = {0.0, -1.0, 1.0, 0.0};
+    double es = 0.0, mm = 0.0;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            es = max_nonneg(es, fabs(fma(P[i + 2], M[1 + 2 * j], P[i] * M[2 * j]) - Om[i + 2 * j]));
+            mm = max_nonneg(mm, fabs(M[i + 2 * j]));
+        }
+    m.det_max = max_nonneg(m.det_max, edet);
+    m.symp_max = max_nonneg(m.symp_max, es);
+    m.M_max = max_nonneg(m.M_max, mm);
+}
 template <class Sys>
 __device__ __forceinline__ void monitor_step(const Sys& sys, const double* x, MonState& m) {
     double M[4];
     dense_tangent(sys, x, M);
-    const double edet = fabs((M[0] * M[3] - M[2] * M[1]) - 1.0);
-    const double Om[4] = {0.0, -1.0, 1.0, 0.0};
-    double P[4], Q[4];
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int i = 0; i < 2; ++i)   // (M')[i, q] = M[q, i]
-            P[i + 2 * j] = fma(M[1 + 2 * i], Om[1 + 2 * j], M[2 * i] * Om[2 * j]);
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int i = 0; i < 2; ++i) Q[i + 2 * j] = fma(P[i + 2], M[1 + 2 * j], P[i] * M[2 * j]);
-    double es = fabs(Q[0] - Om[0]);
-#pragma unroll
-    for (int l = 1; l < 4; ++l) es = jl_max(es, fabs(Q[l] - Om[l]));
-    double mm = fabs(M[0]);
-#pragma unroll
-    for (int l = 1; l < 4; ++l) mm = jl_max(mm, fabs(M[l]));
-    m.det_max = jl_max(m.det_max, edet);
-    m.symp_max = jl_max(m.symp_max, es);
-    m.M_max = jl_max(m.M_max, mm);
+    monitor_tangent(M, m);
+}
+// The same from the tangent entries J of the next step, which the recorders evaluate at this very point: a standard
+// map's sine and cosine are taken once, not twice (mixed kernels hold a Float32 J and take their own).
+template <class Sys, class J>
+__device__ __forceinline__ void monitor_ahead(const Sys& sys, const double* x, const J& Jn, MonState& m) {
+    if constexpr (std::is_same<J, StdJac>::value) {
+        const double M[4] = {1.0 + Jn.c, Jn.c, 1.0, 1.0};
+        monitor_tangent(M, m);
+    } else {
+        monitor_step(sys, x, m);
+    }
 }
 
 }  // namespace cl
