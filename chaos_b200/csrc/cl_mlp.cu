@@ -199,17 +199,15 @@ __device__ __forceinline__ void stage_tile(uint32_t dst, const __nv_bfloat16* __
     }
 }
 
-// C[M x N] (+)= A . B^T: one CTA of 128 threads per 128 x NT output tile and K range (split-K over gridDim.z).
-// STAGES-deep ring of shared-memory stages filled by cp.async; one thread issues the stage's BK / 16 MMAs and
-// commits them to the stage's mbarrier, which the copies into that stage wait on before it is refilled, so the
-// loads of the next STAGES - 1 blocks overlap the tensor cores. With split-K (gridDim.z > 1) the partial tiles are
-// added to C32 with atomics (C32 zeroed by the caller; no bias, epilogue or BF16 output).
-template <int NT, int STAGES>
-__global__ void __launch_bounds__(128, 1) gemm_bf16_tc(const __nv_bfloat16* __restrict__ A, int lda,
-                                                       const __nv_bfloat16* __restrict__ B, int ldb, int M, int N,
-                                                       int K, const float* __restrict__ bias, int epilogue,
-                                                       float* __restrict__ C32, __nv_bfloat16* __restrict__ Cb,
-                                                       int ldc, float* __restrict__ pre, int accumulate) {
+// One 128 x NT tile of A . B^T over the K blocks kb0..kb1 - 1 by a CTA of 128 threads: a STAGES-deep ring of
+// shared-memory stages filled by cp.async; one thread issues the stage's BK / 16 MMAs and commits them to the stage's
+// mbarrier, which the copies into that stage wait on before it is refilled, so the loads of the next STAGES - 1 blocks
+// overlap the tensor cores. Then `epi(row, c0, r)` for every 16 columns c0 of the tile: r the accumulator's bits of this
+// thread's row (every lane of a warp calls it together; row may be past M).
+template <int NT, int STAGES, class Epilogue>
+__device__ __forceinline__ void gemm_tile(const __nv_bfloat16* __restrict__ A, int lda,
+                                          const __nv_bfloat16* __restrict__ B, int ldb, int m0, int n0, int M, int N,
+                                          int K, int kb0, int kb1, Epilogue&& epi) {
     constexpr int TCOLS = NT < 32 ? 32 : NT;   // TMEM allocation: a power of two, at least 32 columns
     constexpr int A_BYTES = BM * BK * 2, B_BYTES = NT * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
     static_assert((NT % 16) == 0 && NT >= 16 && NT <= 256, "N tile");
@@ -217,14 +215,7 @@ __global__ void __launch_bounds__(128, 1) gemm_bf16_tc(const __nv_bfloat16* __re
     __shared__ __align__(8) uint64_t mbar[STAGES];
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * NT;
-    const int kblocks_all = (K + BK - 1) / BK;
-    const int per = (kblocks_all + gridDim.z - 1) / gridDim.z;
-    const int kb0 = blockIdx.z * per, kb1 = min(kblocks_all, kb0 + per), nkb = max(0, kb1 - kb0);
-    const bool split = gridDim.z > 1;
-    // vector epilogue: rows of C / pre start 32-byte aligned (ldc % 8 == 0 and 32-byte aligned bases)
-    const bool vec = (ldc % 8) == 0 && (reinterpret_cast<uintptr_t>(C32) & 31) == 0 &&
-                     (reinterpret_cast<uintptr_t>(Cb) & 15) == 0 && (reinterpret_cast<uintptr_t>(pre) & 31) == 0;
+    const int nkb = max(0, kb1 - kb0);
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
@@ -320,6 +311,35 @@ __global__ void __launch_bounds__(128, 1) gemm_bf16_tc(const __nv_bfloat16* __re
                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                 : "r"(taddr));
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            epi(row, c0, r);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" :: "r"(tmem), "r"(TCOLS) : "memory");
+    }
+}
+
+// C[M x N] (+)= A . B^T: one CTA per 128 x NT output tile and K range (split-K over gridDim.z). With split-K
+// (gridDim.z > 1) the partial tiles are added to C32 with atomics (C32 zeroed by the caller; no bias, epilogue or BF16
+// output).
+template <int NT, int STAGES>
+__global__ void __launch_bounds__(128, 1) gemm_bf16_tc(const __nv_bfloat16* __restrict__ A, int lda,
+                                                       const __nv_bfloat16* __restrict__ B, int ldb, int M, int N,
+                                                       int K, const float* __restrict__ bias, int epilogue,
+                                                       float* __restrict__ C32, __nv_bfloat16* __restrict__ Cb,
+                                                       int ldc, float* __restrict__ pre, int accumulate) {
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * NT;
+    const int kblocks_all = (K + BK - 1) / BK;
+    const int per = (kblocks_all + gridDim.z - 1) / gridDim.z;
+    const int kb0 = blockIdx.z * per, kb1 = min(kblocks_all, kb0 + per);
+    const bool split = gridDim.z > 1;
+    // vector epilogue: rows of C / pre start 32-byte aligned (ldc % 8 == 0 and 32-byte aligned bases)
+    const bool vec = (ldc % 8) == 0 && (reinterpret_cast<uintptr_t>(C32) & 31) == 0 &&
+                     (reinterpret_cast<uintptr_t>(Cb) & 15) == 0 && (reinterpret_cast<uintptr_t>(pre) & 31) == 0;
+    gemm_tile<NT, STAGES>(A, lda, B, ldb, m0, n0, M, N, K, kb0, kb1, [&](int row, int c0, const uint32_t (&r)[16]) {
             if (row < M) {
                 const int colb = n0 + c0;
                 const size_t at0 = static_cast<size_t>(row) * ldc + colb;
@@ -383,14 +403,7 @@ __global__ void __launch_bounds__(128, 1) gemm_bf16_tc(const __nv_bfloat16* __re
                     }
                 }
             }
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (warp == 0) {
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" :: "r"(tmem), "r"(TCOLS) : "memory");
-    }
+    });
 }
 
 // ---- the fused forward pass --------------------------------------------------------------------------------------
@@ -881,6 +894,231 @@ __global__ void f32_to_bf16(const float* __restrict__ x, int64_t n, __nv_bfloat1
     if (i < n) y[i] = __float2bfloat16(x[i]);
 }
 
+// ---- the training step -------------------------------------------------------------------------------------------
+// One step of the screen network (forward, loss, gradients, Adam) as ten launches on one workspace. What bounded it
+// before was the host: 45 launches and 30 allocations of a few microseconds each from Python, 425 us at the pipeline's
+// batch of 4096 rows, where the arithmetic is 3.5 GFLOP. Each pass now leaves what the next ones read: an activation
+// or a gradient goes out row-major (the next product's operand) and transposed (the weight gradient's, whose
+// contraction runs over the rows), the activation's derivative and the bias gradients' column sums sit in the epilogue
+// of the product that makes them, all weight gradients are one launch over (layer, tile, K range), and the last launch
+// adds their partial tiles in a fixed order and runs Adam on every weight and bias. The products, roundings to BF16 and
+// elementwise operations are those of the per-layer path; only the order of the gradients' sums differs. 4096 rows: 417
+// -> 115 us a step.
+constexpr int T_LAYERS = 4;
+__host__ __device__ constexpr int t_in(int l) { return l == 0 ? 64 : 256; }
+__host__ __device__ constexpr int t_out(int l) { return l == 3 ? 16 : 256; }
+__host__ __device__ constexpr int t_off(int l) { return l == 0 ? 0 : l == 1 ? 16384 : l == 2 ? 81920 : 147456; }
+constexpr int T_WEIGHTS = 151552;
+
+// sums over a warp's rows of 16 columns: lane 2q (and 2q + 1) returns column q's
+__device__ __forceinline__ float warp_columns(float (&v)[16], int lane) {
+#pragma unroll
+    for (int h = 8; h >= 1; h >>= 1) {
+        const bool up = (lane & (2 * h)) != 0;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const float send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * h);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+// a row's 16 values as BF16, row-major (16-byte stores) and transposed (a warp's 32 rows are contiguous there)
+__device__ __forceinline__ void put_bf16(const float (&v)[16], __nv_bfloat16* rowp, __nv_bfloat16* colp, size_t ldt) {
+    uint32_t w[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+        w[q] = *reinterpret_cast<const uint32_t*>(&h);
+        colp[static_cast<size_t>(2 * q) * ldt] = h.x;
+        colp[static_cast<size_t>(2 * q + 1) * ldt] = h.y;
+    }
+    if (rowp) {
+        reinterpret_cast<uint4*>(rowp)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        reinterpret_cast<uint4*>(rowp)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+
+// A hidden layer forward: pre = A W^T + b, H = GELU(pre), H's transpose. Rows are a multiple of 128.
+template <int NT>
+__global__ void __launch_bounds__(128, 1) train_forward(const __nv_bfloat16* A, int K, const __nv_bfloat16* W,
+                                                        const float* bias, int rows, float* pre, __nv_bfloat16* H,
+                                                        __nv_bfloat16* Ht) {
+    const int n0 = blockIdx.y * NT;
+    gemm_tile<NT, 3>(A, K, W, K, blockIdx.x * BM, n0, rows, 256, K, 0, (K + BK - 1) / BK,
+                     [&](int row, int c0, const uint32_t (&r)[16]) {
+        float v[16];
+        const int col = n0 + c0;
+        const size_t at = static_cast<size_t>(row) * 256 + col;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + bias[col + j];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            reinterpret_cast<float4*>(pre + at)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = gelu_t(v[j]);
+        put_bf16(v, H + at, Ht + static_cast<size_t>(col) * rows + row, rows);
+    });
+}
+
+// The head: its 16 outputs, the row's loss and gradient (head_loss's operations), the column sums per 128 rows.
+__global__ void __launch_bounds__(128, 1) train_head(const __nv_bfloat16* A, const __nv_bfloat16* W, const float* bias,
+                                                     int rows, const float* label, const float* target, float w_reg,
+                                                     float* row_loss, __nv_bfloat16* G, __nv_bfloat16* Gt,
+                                                     float* colsum) {
+    __shared__ float cs[4][16];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    gemm_tile<16, 3>(A, 256, W, 256, blockIdx.x * BM, 0, rows, 16, 256, 0, 256 / BK,
+                     [&](int row, int, const uint32_t (&r)[16]) {
+        float g[16];
+        const float z = __uint_as_float(r[0]) + bias[0], lam = __uint_as_float(r[1]) + bias[1], y = label[row];
+        const float p = 1.0f / (1.0f + __expf(-z));
+        const float bce = fmaxf(z, 0.f) - z * y + log1pf(__expf(-fabsf(z)));
+        const float e = lam - target[row];
+        row_loss[row] = bce + w_reg * e * e;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) g[j] = 0.f;
+        g[0] = (p - y) / rows;
+        g[1] = 2.0f * w_reg * e / rows;
+        put_bf16(g, G + static_cast<size_t>(row) * 16, Gt + row, rows);
+        const float s = warp_columns(g, lane);
+        if (!(lane & 1)) cs[warp][lane >> 1] = s;
+    });
+    __syncthreads();
+    if (threadIdx.x < 16)
+        colsum[blockIdx.x * 16 + threadIdx.x] = (cs[0][threadIdx.x] + cs[1][threadIdx.x]) + (cs[2][threadIdx.x] + cs[3][threadIdx.x]);
+}
+
+// A hidden layer backward: dZ = (dZ_next W_next) GELU'(pre), in BF16 both ways, and its column sums per 128 rows.
+template <int NT>
+__global__ void __launch_bounds__(128, 1) train_backward(const __nv_bfloat16* G, int K, const __nv_bfloat16* Wt,
+                                                         const float* pre, int rows, __nv_bfloat16* D,
+                                                         __nv_bfloat16* Dt, float* colsum) {
+    __shared__ float cs[4][NT];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n0 = blockIdx.y * NT;
+    gemm_tile<NT, 3>(G, K, Wt, K, blockIdx.x * BM, n0, rows, 256, K, 0, (K + BK - 1) / BK,
+                     [&](int row, int c0, const uint32_t (&r)[16]) {
+        float v[16];
+        const int col = n0 + c0;
+        const size_t at = static_cast<size_t>(row) * 256 + col;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 z = reinterpret_cast<const float4*>(pre + at)[q];
+            v[4 * q] = __fmul_rn(__uint_as_float(r[4 * q]), gelu_t_grad(z.x));
+            v[4 * q + 1] = __fmul_rn(__uint_as_float(r[4 * q + 1]), gelu_t_grad(z.y));
+            v[4 * q + 2] = __fmul_rn(__uint_as_float(r[4 * q + 2]), gelu_t_grad(z.z));
+            v[4 * q + 3] = __fmul_rn(__uint_as_float(r[4 * q + 3]), gelu_t_grad(z.w));
+        }
+        put_bf16(v, D ? D + at : nullptr, Dt + static_cast<size_t>(col) * rows + row, rows);
+        const float s = warp_columns(v, lane);
+        if (!(lane & 1)) cs[warp][c0 + (lane >> 1)] = s;
+    });
+    __syncthreads();
+    for (int c = threadIdx.x; c < NT; c += 128)
+        colsum[static_cast<size_t>(blockIdx.x) * 256 + n0 + c] = (cs[0][c] + cs[1][c]) + (cs[2][c] + cs[3][c]);
+}
+
+// All weight gradients: blockIdx.x a (layer, 128 x 64 tile), blockIdx.y a range of the rows; partial tiles side by side.
+struct TrainGrads { const __nv_bfloat16* Dt[T_LAYERS]; const __nv_bfloat16* At[T_LAYERS]; float* part; int rows; };
+constexpr int T_TILES = 22;   // 2 x 1, 2 x 4, 2 x 4, 1 x 4
+__global__ void __launch_bounds__(128, 1) train_weight_grads(const TrainGrads a) {
+    const int t = blockIdx.x, l = t < 2 ? 0 : t < 10 ? 1 : t < 18 ? 2 : 3;
+    const int q = t - (l == 0 ? 0 : l == 1 ? 2 : l == 2 ? 10 : 18);
+    const int M = t_out(l), N = t_in(l), nt = N / 64, m0 = (q / nt) * BM, n0 = (q % nt) * 64;
+    const int kblocks = a.rows / BK, per = (kblocks + gridDim.y - 1) / gridDim.y;
+    const int kb0 = min(kblocks, static_cast<int>(blockIdx.y) * per), kb1 = min(kblocks, kb0 + per);
+    float* out = a.part + static_cast<size_t>(blockIdx.y) * T_WEIGHTS + t_off(l);
+    gemm_tile<64, 3>(a.Dt[l], a.rows, a.At[l], a.rows, m0, n0, M, N, a.rows, kb0, kb1,
+                     [&](int row, int c0, const uint32_t (&r)[16]) {
+        if (row >= M) return;
+        float4* o = reinterpret_cast<float4*>(out + static_cast<size_t>(row) * N + n0 + c0);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            o[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
+                               __uint_as_float(r[4 * j + 3]));
+    });
+}
+
+struct TrainLayer { float *W, *b; __nv_bfloat16 *Wb, *Wbt; float *mW, *vW, *mb, *vb, *gW, *gb; };
+struct TrainUpdate {
+    TrainLayer layer[T_LAYERS];
+    const float* part;              // splits x T_WEIGHTS
+    const float* colsum[T_LAYERS];  // tiles x outputs
+    int splits, tiles;
+    float lr, b1, b2, eps, c1, c2;
+};
+__device__ __forceinline__ float adam_value(float w, float g, float* m, float* v, const TrainUpdate& a) {
+    const float mi = a.b1 * *m + (1.0f - a.b1) * g, vi = a.b2 * *v + (1.0f - a.b2) * g * g;
+    *m = mi;
+    *v = vi;
+    return w - a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+}
+// The partial gradients summed in their order, then Adam (adam_step's operations): blocks of 256 weights, then one block
+// per 32 biases (8 row lanes over the 128-row sums, folded in shared memory).
+constexpr int T_WBLOCKS = T_WEIGHTS / 256, T_BBLOCKS = 25;
+__global__ void __launch_bounds__(256) train_update(const TrainUpdate a) {
+    if (blockIdx.x < T_WBLOCKS) {
+        const int i = blockIdx.x * 256 + threadIdx.x;
+        const int l = i < t_off(1) ? 0 : i < t_off(2) ? 1 : i < t_off(3) ? 2 : 3;
+        const TrainLayer& y = a.layer[l];
+        const int e = i - t_off(l), N = t_in(l), r = e / N, c = e % N;
+        float g = a.part[i];
+        for (int s = 1; s < a.splits; ++s) g += a.part[static_cast<size_t>(s) * T_WEIGHTS + i];
+        y.gW[e] = g;
+        const float w = adam_value(y.W[e], g, y.mW + e, y.vW + e, a);
+        y.W[e] = w;
+        const __nv_bfloat16 h = __float2bfloat16(w);
+        y.Wb[e] = h;
+        y.Wbt[static_cast<size_t>(c) * t_out(l) + r] = h;
+        return;
+    }
+    __shared__ float sum[8][32];
+    const int j = blockIdx.x - T_WBLOCKS, lane = threadIdx.x & 31, rl = threadIdx.x >> 5;
+    const int l = j >> 3, c = (j & 7) * 32 + lane, n = t_out(l);   // layers of 8, 8, 8 and 1 blocks
+    float s = 0.f;
+    if (c < n)
+        for (int t = rl; t < a.tiles; t += 8) s += a.colsum[l][static_cast<size_t>(t) * n + c];
+    sum[rl][lane] = s;
+    __syncthreads();
+    if (rl == 0 && c < n) {
+        float g = sum[0][lane];
+        for (int q = 1; q < 8; ++q) g += sum[q][lane];
+        const TrainLayer& y = a.layer[l];
+        y.gb[c] = g;
+        y.b[c] = adam_value(y.b[c], g, y.mb + c, y.vb + c, a);
+    }
+}
+
+// The step's workspace: byte offsets of its arrays (each a multiple of 256) for `rows` rows and `splits` K ranges.
+struct TrainSpace {
+    size_t Xt, H[3], Ht[3], pre[3], G, Gt, D[3], Dt[3], colsum[T_LAYERS], part, bytes;
+};
+TrainSpace train_space(int64_t rows, int splits) {
+    TrainSpace w;
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) / 256 * 256; return o; };
+    const size_t n = static_cast<size_t>(rows);
+    w.Xt = take(n * 64 * 2);
+    for (int l = 0; l < 3; ++l) { w.H[l] = take(n * 512); w.Ht[l] = take(n * 512); w.pre[l] = take(n * 1024); }
+    w.G = take(n * 32);
+    w.Gt = take(n * 32);
+    for (int l = 0; l < 3; ++l) { w.D[l] = take(n * 512); w.Dt[l] = take(n * 512); }
+    for (int l = 0; l < T_LAYERS; ++l) w.colsum[l] = take(n / 128 * t_out(l) * 4);
+    w.part = take(static_cast<size_t>(splits) * T_WEIGHTS * 4);
+    w.bytes = at;
+    return w;
+}
+// K ranges of the weight gradients: at least 8 blocks of 64 rows each, up to about two tiles an SM
+int train_splits(int64_t rows) {
+    const int64_t kblocks = rows / BK, most = std::max<int64_t>(1, std::min<int64_t>(kblocks / 8, 13));
+    const int64_t per = (kblocks + most - 1) / most;
+    return static_cast<int>((kblocks + per - 1) / per);   // no range is empty
+}
+template <class K>
+cudaError_t train_smem(K k, int nt) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * (BM + nt) * BK * 2);
+}
+
 template <int NT>
 cudaError_t launch_gemm(const void* A, int lda, const void* B, int ldb, int M, int N, int K, const float* bias,
                         int epi, float* C32, void* Cb, int ldc, float* pre, int acc, int splits, cudaStream_t st) {
@@ -1010,6 +1248,76 @@ int cl_b200_mlp_forward_fused(const void* X, int32_t B, const void* Wp1, const v
     capi_count_launch();
     e = cudaGetLastError();
     return e == cudaSuccess ? 0 : capi_map_cuda(e, "fused forward launch");
+}
+
+int64_t cl_b200_mlp_train_workspace(int32_t B) {
+    return B > 0 && B % BM == 0 ? static_cast<int64_t>(train_space(B, train_splits(B)).bytes) : 0;
+}
+
+int cl_b200_mlp_train_step(const void* X, int32_t B, const void* const* layers, const float* label, const float* target,
+                           float w_reg, float lr, float b1, float b2, float eps, int32_t t, void* workspace,
+                           int64_t workspace_bytes, float* row_loss, void* stream) {
+    if (!X || !layers || !label || !target || !workspace || !row_loss || B <= 0 || B % BM || t < 1)
+        return capi_fail(CL_EINVAL, "train step: bad arguments (a batch is a positive multiple of 128 rows)");
+    for (int i = 0; i < 10 * T_LAYERS; ++i)
+        if (!layers[i] || reinterpret_cast<uintptr_t>(layers[i]) % 16)
+            return capi_fail(CL_EINVAL, "train step: every layer array needs 16-byte alignment");
+    const int splits = train_splits(B);
+    const TrainSpace w = train_space(B, splits);
+    if (workspace_bytes < static_cast<int64_t>(w.bytes) || reinterpret_cast<uintptr_t>(workspace) % 256 ||
+        reinterpret_cast<uintptr_t>(X) % 16)
+        return capi_fail(CL_EINVAL, "train step: workspace too small, or it or X misaligned");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    uint8_t* base = static_cast<uint8_t*>(workspace);
+    auto bf = [&](size_t o) { return reinterpret_cast<__nv_bfloat16*>(base + o); };
+    auto fp = [&](size_t o) { return reinterpret_cast<float*>(base + o); };
+    TrainUpdate u;
+    for (int l = 0; l < T_LAYERS; ++l) {
+        void* const* p = const_cast<void* const*>(layers) + 10 * l;
+        TrainLayer& y = u.layer[l];
+        y.W = static_cast<float*>(p[0]); y.b = static_cast<float*>(p[1]);
+        y.Wb = static_cast<__nv_bfloat16*>(p[2]); y.Wbt = static_cast<__nv_bfloat16*>(p[3]);
+        y.mW = static_cast<float*>(p[4]); y.vW = static_cast<float*>(p[5]); y.mb = static_cast<float*>(p[6]);
+        y.vb = static_cast<float*>(p[7]); y.gW = static_cast<float*>(p[8]); y.gb = static_cast<float*>(p[9]);
+        u.colsum[l] = fp(w.colsum[l]);
+    }
+    u.part = fp(w.part);
+    u.splits = splits;
+    u.tiles = B / BM;
+    u.lr = lr; u.b1 = b1; u.b2 = b2; u.eps = eps;
+    u.c1 = 1.0f - powf(b1, static_cast<float>(t));
+    u.c2 = 1.0f - powf(b2, static_cast<float>(t));
+    // 64-column tiles while 128-column ones would leave SMs without a tile
+    const bool narrow = u.tiles * 2 < 2 * 148;
+    const int nt = narrow ? 64 : 128, sm64 = 3 * (BM + 64) * BK * 2, smn = 3 * (BM + nt) * BK * 2, sm16 = 3 * (BM + 16) * BK * 2;
+    auto fwd = narrow ? train_forward<64> : train_forward<128>;
+    auto bwd = narrow ? train_backward<64> : train_backward<128>;
+    cudaError_t e;
+    if ((e = train_smem(fwd, nt)) != cudaSuccess || (e = train_smem(bwd, nt)) != cudaSuccess ||
+        (e = train_smem(train_head, 16)) != cudaSuccess || (e = train_smem(train_weight_grads, 64)) != cudaSuccess)
+        return capi_map_cuda(e, "train step setup");
+    const dim3 grid(u.tiles, 256 / nt);
+    transpose_bf16<<<dim3(2, (B + 31) / 32), dim3(32, 8), 0, st>>>(static_cast<const __nv_bfloat16*>(X), B, 64, 64, bf(w.Xt), B);
+    const __nv_bfloat16* in = static_cast<const __nv_bfloat16*>(X);
+    for (int l = 0; l < 3; ++l) {
+        fwd<<<grid, 128, smn, st>>>(in, t_in(l), u.layer[l].Wb, u.layer[l].b, B, fp(w.pre[l]), bf(w.H[l]), bf(w.Ht[l]));
+        in = bf(w.H[l]);
+    }
+    train_head<<<u.tiles, 128, sm16, st>>>(in, u.layer[3].Wb, u.layer[3].b, B, label, target, w_reg, row_loss, bf(w.G),
+                                           bf(w.Gt), fp(w.colsum[3]));
+    const __nv_bfloat16* g = bf(w.G);
+    for (int l = 2; l >= 0; --l) {
+        bwd<<<grid, 128, smn, st>>>(g, t_out(l + 1), u.layer[l + 1].Wbt, fp(w.pre[l]), B, l > 0 ? bf(w.D[l]) : nullptr,
+                                    bf(w.Dt[l]), fp(w.colsum[l]));
+        g = bf(w.D[l]);
+    }
+    const TrainGrads tg{{bf(w.Dt[0]), bf(w.Dt[1]), bf(w.Dt[2]), bf(w.Gt)}, {bf(w.Xt), bf(w.Ht[0]), bf(w.Ht[1]), bf(w.Ht[2])},
+                        fp(w.part), B};
+    train_weight_grads<<<dim3(T_TILES, splits), 128, sm64, st>>>(tg);
+    train_update<<<T_WBLOCKS + T_BBLOCKS, 256, 0, st>>>(u);
+    for (int i = 0; i < 10; ++i) capi_count_launch();
+    e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : capi_map_cuda(e, "train step launch");
 }
 
 int cl_b200_mlp_status(void) {

@@ -44,7 +44,11 @@ def _declare(L):
     L.cl_b200_mlp_status.argtypes = []
     L.cl_b200_mlp_pack_kmajor.argtypes = [vp, C.c_int32, C.c_int32, C.c_int32, C.c_int32, vp, vp]
     L.cl_b200_mlp_forward_fused.argtypes = [vp, C.c_int32, vp, vp, vp, vp, f32p, f32p, f32p, f32p, f32p, C.c_int32, vp]
-    for nm in ("cl_b200_mlp_pack_kmajor", "cl_b200_mlp_forward_fused", "cl_b200_gemm_bf16", "cl_b200_transpose_bf16", "cl_b200_gelu_backward", "cl_b200_col_sum",
+    L.cl_b200_mlp_train_workspace.argtypes = [C.c_int32]
+    L.cl_b200_mlp_train_workspace.restype = C.c_int64
+    L.cl_b200_mlp_train_step.argtypes = [vp, C.c_int32, C.POINTER(vp), f32p, f32p] + [C.c_float] * 5 + \
+        [C.c_int32, vp, C.c_int64, f32p, vp]
+    for nm in ("cl_b200_mlp_train_step", "cl_b200_mlp_pack_kmajor", "cl_b200_mlp_forward_fused", "cl_b200_gemm_bf16", "cl_b200_transpose_bf16", "cl_b200_gelu_backward", "cl_b200_col_sum",
                "cl_b200_head_loss", "cl_b200_adam", "cl_b200_to_bf16", "cl_b200_screen_features",
                "cl_b200_mlp_status"):
         getattr(L, nm).restype = C.c_int
@@ -240,6 +244,22 @@ class MLP:
                                self.stream()), "adam b")
 
     def train_step(self, Xb, label, target, w_reg=1.0, lr=1e-3):
+        """Forward, loss, gradients (in each layer's gW, gb) and Adam on one batch; returns the row losses. Batches of
+        whole 128-row tiles run as one native call (ten launches); others pass by pass."""
+        B = Xb.shape[0]
+        if self.dims == DIMS and B % 128 == 0 and B:
+            t, L = self.t, _declare(lib())
+            Xb, label, target = Xb.contiguous(), label.contiguous(), target.contiguous()
+            nbytes = L.cl_b200_mlp_train_workspace(B)
+            ws = t.empty(nbytes, dtype=t.uint8, device=self.dev)
+            rl = t.empty(B, dtype=t.float32, device=self.dev)
+            ptrs = (C.c_void_p * 40)(*[lay[k].data_ptr() for lay in self.layers
+                                       for k in ("W", "b", "Wb", "Wbt", "mW", "vW", "mb", "vb", "gW", "gb")])
+            _ck(L.cl_b200_mlp_train_step(Xb.data_ptr(), B, ptrs, label.data_ptr(), target.data_ptr(), w_reg, lr, 0.9,
+                                         0.999, 1e-8, self.step + 1, ws.data_ptr(), nbytes, rl.data_ptr(),
+                                         self.stream()), "train step")
+            self.step += 1
+            return rl
         out = self.forward(Xb, keep=True)
         rl, g32, gb = self.loss_and_grad(out, label, target, w_reg)
         self.backward(g32, gb)

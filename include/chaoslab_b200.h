@@ -460,6 +460,15 @@ CL_API int cl_b200_mlp_forward_fused(const void* X, int32_t B, const void* Wp1, 
                                      const float* b4, float* out, int32_t max_ctas, void* stream);
 /* 0, or CL_EDEVICE_LOST after a bounded wait on an MMA or copy barrier (GEMM or fused pass) gave up. */
 CL_API int cl_b200_mlp_status(void);
+/* One training step of that network: forward, mean binary cross-entropy on `label` plus w_reg times the mean squared
+ * error on `target`, gradients, Adam (step count t), with the row losses in row_loss. B is a multiple of 128; `layers`
+ * holds, for each of the four layers in order, the device pointers {W, b, W in BF16, its transpose in BF16, Adam's m and
+ * v of W, m and v of b, the gradients of W and b} (FP32 but the BF16 copies; the last layer's 2 outputs padded to 16).
+ * `workspace`: cl_b200_mlp_train_workspace(B) bytes, 256-byte aligned, free again when the stream has passed the call. */
+CL_API int64_t cl_b200_mlp_train_workspace(int32_t B);
+CL_API int cl_b200_mlp_train_step(const void* X, int32_t B, const void* const* layers, const float* label,
+                                  const float* target, float w_reg, float lr, float b1, float b2, float eps, int32_t t,
+                                  void* workspace, int64_t workspace_bytes, float* row_loss, void* stream);
 CL_API int cl_b200_transpose_bf16(const void* src, int32_t rows, int32_t cols, int32_t lds, void* dst, int32_t ldd,
                                   void* stream);
 /* dH = dY * GELU'(pre), to BF16 (dHb) and / or FP32 (dH32). */
