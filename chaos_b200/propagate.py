@@ -25,6 +25,7 @@ from .systems import System
 
 STATUS_OK, STATUS_STATE, STATUS_W, STATUS_REDUCER = 0, 1, 2, 3
 CHUNK_HEADROOM = 0.5
+PROBE_BYTES = 1 << 30   # device bytes of a run below which its chunk is not sized by the free memory beforehand
 PRECISIONS = {"fp64": _abi.PREC_FP64, "mixed": _abi.PREC_MIXED, "mixed-ind64": _abi.PREC_MIXED_IND64}
 PRECISION_LABELS = {"fp64": "Float64", "mixed": "Float64 orbit / Float32 tangent",
                     "mixed-ind64": "Float64 orbit and indicator frames / Float32 Lyapunov frames"}
@@ -204,12 +205,16 @@ def propagate_frames(sys: System, x0, N: int, frames: list[FrameSpec], *, tau: i
     run.steps = Lsteps
     dtypes = [chain_dtype(fr.reducers, d, fr.k) for fr in frames]
     rbytes = sum(dt.itemsize for dt in dtypes)
-    if chunk is None:
-        pr = probe()
-        kk = max(fr.k for fr in frames)
-        csize = chunk_size(pr["free_bytes"], d, kk, reducer_bytes=rbytes, s=s) if pr["free_bytes"] else n
-    else:
-        csize = chunk
+    kk = max(fr.k for fr in frames)
+
+    def probed_chunk():
+        free = probe()["free_bytes"]
+        return chunk_size(free, d, kk, reducer_bytes=rbytes, s=s) if free else n
+
+    # Asking the driver for the free memory takes 0.2 ms, and tens of milliseconds beside other processes' work; a run
+    # of less than PROBE_BYTES is tried whole, and asks only if its allocation fails.
+    unprobed = chunk is None and n * (bytes_per_orbit(d, kk, s) + rbytes) <= PROBE_BYTES
+    csize = chunk if chunk is not None else (n if unprobed else probed_chunk())
     csize = min(csize, cap, n) if n else 1
     x = np.empty((n, s))
     Wout = [np.empty((n, fr.k, d)) for fr in frames]
@@ -219,7 +224,8 @@ def propagate_frames(sys: System, x0, N: int, frames: list[FrameSpec], *, tau: i
     prov_dev = _abi.cl_prov()
     gpu_ms, chunks = 0.0, 0
     errors: list = [None] * len(frames)
-    for lo in range(0, n, csize):
+    lo = 0
+    while lo < n:
         hi = min(lo + csize, n)
         run.orbit_base = lo
         bufs = _abi.cl_buffers()
@@ -234,6 +240,12 @@ def propagate_frames(sys: System, x0, N: int, frames: list[FrameSpec], *, tau: i
         hook = launch_plan.BEFORE_LAUNCH
         if hook is None:   # every launch of the chunk inside one library call
             rc = L.cl_b200_propagate(C.byref(run), hi - lo, C.byref(bufs), C.byref(prov_dev))
+            if rc == _abi.ENOMEM and unprobed:
+                msg, unprobed = last_error(), False
+                if probed_chunk() >= csize:
+                    raise DeviceError(rc, msg)
+                csize = max(1, min(probed_chunk(), csize))
+                continue
             if rc != 0:
                 raise DeviceError(rc, last_error())
             gpu_ms += prov_dev.gpu_ms
@@ -253,6 +265,7 @@ def propagate_frames(sys: System, x0, N: int, frames: list[FrameSpec], *, tau: i
                     errors[f] = _reducer_error(tuple(fr.reducers), states[f][i], i + 1, "gpu")
                 else:
                     errors[f] = _health_error(c, x[i], Wout[f][i].T, int(hsteps[f][i]), i + 1, "gpu")
+        lo = hi
     if throw:
         for e in errors:
             if e is not None:

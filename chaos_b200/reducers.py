@@ -20,6 +20,15 @@ def _cs(name):
     return [(name + "_s", "<f8"), (name + "_c", "<f8")]
 
 
+def _words(field, *shape):
+    """The Float64 words that follow a state's field, as a view: `shape` numbers them row-major within the record."""
+    strides, step = [], 8
+    for k in reversed(shape):
+        strides.insert(0, step)
+        step *= k
+    return np.lib.stride_tricks.as_strided(field, (len(field), *shape), (field.strides[0], *strides))
+
+
 def _tot(s, c):
     return float(np.float64(s) + np.float64(c))
 
@@ -190,8 +199,8 @@ class SALI(Reducer):
 
     def finals(self, st, d=None):
         n = st["n"].astype(np.int64, copy=False)
-        s = np.stack([st["s1_s"], st["s2_s"]], axis=1).astype(np.float64, copy=False)
-        c = np.stack([st["s1_c"], st["s2_c"]], axis=1).astype(np.float64, copy=False)
+        v = _words(st["s1_s"], 2, 2)   # (column, sum / comp)
+        s, c = v[:, :, 0], v[:, :, 1]
         L = np.where(n == 0, 0.0, -((s[:, 0] + s[:, 1]) + (c[:, 0] + c[:, 1])))
         return dict(n=n, sali=st["sali"].astype(np.float64, copy=False), L=L, sum=s, comp=c, floor=np.full(len(n), 4 * EPS))
 
@@ -307,24 +316,19 @@ class MEGNO(Reducer):
                     sum=pair("s", "s"), comp=pair("s", "c"), R1=tot("R1"), R2=tot("R2"), Q=tot("Q"), Q2=tot("Q2"))
 
     def finals(self, st, d=None):
+        # (column, s R1 R2 Q Q2, sum / comp): one pass for every total instead of one per field
         n, K = st["n"].astype(np.int64, copy=False), st["K"].astype(np.int64, copy=False)
-        f = np.float64
-        tn = n.astype(f, copy=False)
-        cols = {nm: np.zeros((len(n), 2)) for nm in ("Y", "Ybar", "Ybar20")}
+        v = _words(st["c1_s_s"], 2, 5, 2)
+        tot = v[..., 0] + v[..., 1]
+        tn, zero = n.astype(np.float64)[:, None], (K == 0)[:, None]
         with np.errstate(invalid="ignore", divide="ignore"):
-            nk = np.where(K == 0, 0, n // np.where(K == 0, 1, K)).astype(f, copy=False)
-            for j, col in enumerate(("c1", "c2")):
-                R1 = st[f"{col}_R1_s"].astype(f, copy=False) + st[f"{col}_R1_c"].astype(f, copy=False)
-                Q = st[f"{col}_Q_s"].astype(f, copy=False) + st[f"{col}_Q_c"].astype(f, copy=False)
-                Q2 = st[f"{col}_Q2_s"].astype(f, copy=False) + st[f"{col}_Q2_c"].astype(f, copy=False)
-                cols["Y"][:, j] = np.where(K == 0, 0.0, 2 * R1 / tn)
-                cols["Ybar"][:, j] = np.where(K == 0, 0.0, Q / K.astype(f, copy=False))
-                cols["Ybar20"][:, j] = np.where(K == 0, 0.0, nk * Q2 / (tn * tn * tn))
-        pair = lambda nm, comp: np.stack([st[f"c1_{nm}_{comp}"], st[f"c2_{nm}_{comp}"]], axis=1).astype(f, copy=False)  # noqa
-        tot = lambda nm: np.stack([st[f"c1_{nm}_s"].astype(f, copy=False) + st[f"c1_{nm}_c"].astype(f, copy=False),  # noqa
-                                   st[f"c2_{nm}_s"].astype(f, copy=False) + st[f"c2_{nm}_c"].astype(f, copy=False)], axis=1)
-        return dict(n=n, handoffs=K, Y=cols["Y"], Ybar=cols["Ybar"], Ybar20=cols["Ybar20"], sum=pair("s", "s"),
-                    comp=pair("s", "c"), R1=tot("R1"), R2=tot("R2"), Q=tot("Q"), Q2=tot("Q2"))
+            safe = np.where(K == 0, 1, K)
+            nk = np.where(K == 0, 0, n // safe).astype(np.float64)[:, None]
+            Y = np.where(zero, 0.0, 2 * tot[:, :, 1] / tn)
+            Ybar = np.where(zero, 0.0, tot[:, :, 3] / K.astype(np.float64)[:, None])
+            Ybar20 = np.where(zero, 0.0, nk * tot[:, :, 4] / (tn * tn * tn))
+        return dict(n=n, handoffs=K, Y=Y, Ybar=Ybar, Ybar20=Ybar20, sum=v[:, :, 0, 0], comp=v[:, :, 0, 1],
+                    R1=tot[:, :, 1], R2=tot[:, :, 2], Q=tot[:, :, 3], Q2=tot[:, :, 4])
 
     def error(self, st, orbit, backend):
         v = float(st["value"])
@@ -365,9 +369,9 @@ class FLI(Reducer):
                     stepB=int(st["stepB"]), colB=int(st["colB"]), step1=int(st["step1"]))
 
     def finals(self, st, d=None):
+        v = _words(st["s1_s"], 2, 2)   # (column, sum / comp)
         return dict(n=st["n"].astype(np.int64, copy=False), fli=st["fB"].astype(np.float64, copy=False), fli1=st["f1"].astype(np.float64, copy=False),
-                    sum=np.stack([st["s1_s"], st["s2_s"]], axis=1).astype(np.float64, copy=False),
-                    comp=np.stack([st["s1_c"], st["s2_c"]], axis=1).astype(np.float64, copy=False),
+                    sum=v[:, :, 0], comp=v[:, :, 1],
                     stepB=st["stepB"].astype(np.int64, copy=False), colB=st["colB"].astype(np.int64, copy=False),
                     step1=st["step1"].astype(np.int64, copy=False))
 
