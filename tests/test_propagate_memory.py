@@ -1,12 +1,15 @@
 """A run that was not sized by the free memory beforehand is chunked by it once its allocation fails."""
 from __future__ import annotations
 
+import importlib
+
 import numpy as np
 import pytest
 
-import chaos_b200.propagate as P
 from chaos_b200 import MGS, QRSpectrum, StandardMap, _abi
 from chaos_b200.foundation import DeviceError
+
+P = importlib.import_module("chaos_b200.propagate")   # the package exports a function of that name
 
 
 class _Library:
