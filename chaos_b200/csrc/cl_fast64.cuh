@@ -45,16 +45,19 @@ struct Ok {
     }
 };
 
+// RN(1 / b) from y within an ulp of it (the last step of rcp64)
+__device__ __forceinline__ double rcp64_last(double b, double y) {
+    y = fma(fma(-b, y, 1.0), y, y);
+    const int hb = __double2hiint(b);
+    const bool ones = __double2loint(b) == -1 && (hb & 0xfffff) == 0xfffff;
+    return ones ? __hiloint2double((2046 << 20) - (hb & 0x7ff00000) - (1 << 20), 1) : y;
+}
 // RN(1 / b) for a positive b with an exponent within +-900.
 __device__ __forceinline__ double rcp64(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
     const double e = fma(-b, y, 1.0);
-    y = fma(fma(e, e, e), y, y);
-    y = fma(fma(-b, y, 1.0), y, y);
-    const int hb = __double2hiint(b);
-    const bool ones = __double2loint(b) == -1 && (hb & 0xfffff) == 0xfffff;
-    return ones ? __hiloint2double((2046 << 20) - (hb & 0x7ff00000) - (1 << 20), 1) : y;
+    return rcp64_last(b, fma(fma(e, e, e), y, y));
 }
 // RN(a / b), y = rcp64(b), b > 0; quo64z may give a zero quotient of a zero dividend the other sign
 __device__ __forceinline__ double quo64z(double a, double b, double y) {
@@ -65,17 +68,19 @@ __device__ __forceinline__ double quo64(double a, double b, double y) {
     const double r = quo64z(a, b, y);
     return __hiloint2double(__double2hiint(r) | (__double2hiint(a) & 0x80000000), __double2loint(r));
 }
-// RN(sqrt(s)) for a positive s with an exponent within +-900.
-__device__ __forceinline__ double root64(double s) {
+// RN(sqrt(s)) for a positive s with an exponent within +-900; h: 1 / (2 sqrt(s)) to about an ulp
+__device__ __forceinline__ double root64(double s, double& h) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
-    double g = s * y, h = 0.5 * y;
+    double g = s * y;
+    h = 0.5 * y;
     const double r = fma(-g, h, 0.5);
     const double t = fma(1.5 * r, r, r);
     g = fma(t, g, g);
     h = fma(t, h, h);
     return fma(fma(-g, g, s), h, g);
 }
+__device__ __forceinline__ double root64(double s) { double h; return root64(s, h); }
 // cl_log of a positive normal x, bit for bit, without its special cases
 __device__ __forceinline__ double log64(double x) {
     const int hx = __double2hiint(x);
@@ -107,8 +112,11 @@ __device__ __forceinline__ double log64(double x) {
 // safe_norm<N> of v[0], v[stride], ...: max, quotients by it, the root of their squares' sum. A quotient below 2^-100
 // need not be exact: its square is absorbed by the sum, which holds a 1 when it is complete, whatever its bits.
 // Only the first n <= N entries count (n a constant of the caller's unrolled loop).
+// norm64r also gives the norm's rounded reciprocal: the product of the two reciprocals at hand, 1/m and 1/sqrt of the
+// sum, is within some ulps of it, so one Newton step replaces the hardware estimate and its cubic refinement (30 of 85
+// cycles of the chain).
 template <int N>
-__device__ __forceinline__ double norm64(const double* v, Ok& ok, int n = N) {
+__device__ __forceinline__ double norm64r(const double* v, Ok& ok, double& rcp, int n = N) {
     double t[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) t[i] = i < n ? fabs(v[i]) : 0.0;
@@ -125,7 +133,16 @@ __device__ __forceinline__ double norm64(const double* v, Ok& ok, int n = N) {
 #pragma unroll
     for (int i = 1; i < N; ++i) if (i < n) { q = quo64z(v[i], m, y); s = s + q * q; }
     ok.positive<10>(s);   // in [1, N (1 + eps)]; a NaN among the entries shows here
-    return m * root64(s);
+    double h;
+    const double r = m * root64(s, h);
+    const double e = y * (h + h);
+    rcp = rcp64_last(r, fma(fma(-r, e, 1.0), e, e));
+    return r;
+}
+template <int N>
+__device__ __forceinline__ double norm64(const double* v, Ok& ok, int n = N) {
+    double rcp;   // not used: the compiler drops it
+    return norm64r<N>(v, ok, rcp, n);
 }
 
 // ---- the orthonormalisations of cl_qr.cuh in the straight-line operations ------------------------------------------
@@ -211,7 +228,8 @@ __device__ __forceinline__ void gs64(const double* W, double* Q, double* R, doub
 #pragma unroll
             for (int l = 0; l < D; ++l) u[l] = u[l] - c * qi[l];
         }
-        const double gamma = norm64<D>(u, ok), y = rcp64(gamma);
+        double y;
+        const double gamma = norm64r<D>(u, ok, y);
         R[m + m * K] = gamma;
         rin[m] = y;
 #pragma unroll
@@ -238,7 +256,8 @@ __device__ __forceinline__ int householder64(const double* W, double* Q, double*
         const double c = norm64<D>(a, ok, D - j);
         const bool neg = a[0] < 0.0;
         a[0] = a[0] + (neg ? -c : c);
-        const double nv = norm64<D>(a, ok, D - j), y = rcp64(nv);
+        double y;
+        const double nv = norm64r<D>(a, ok, y, D - j);
 #pragma unroll
         for (int i = 0; i < D; ++i)
             if (i + j < D) {
@@ -308,7 +327,8 @@ __device__ __forceinline__ int givens64(const double* W, double* Q, double* R, d
         for (int i = D - 1; i >= 1; --i) {
             if (i < j + 1) continue;
             const double ab[2] = {rows[i - 1][j], rows[i][j]};
-            const double rho = norm64<2>(ab, ok), y = rcp64(rho);
+            double y;
+            const double rho = norm64r<2>(ab, ok, y);
             ok.dividend(ab[0]);
             ok.dividend(ab[1]);
             const double c = quo64(ab[0], rho, y), s = quo64(ab[1], rho, y);
@@ -402,8 +422,7 @@ __device__ __forceinline__ void pair64(const double* W, Pair64& m) {
     Ok ok;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-        m.a[j] = norm64<D>(W + j * D, ok);
-        m.y[j] = rcp64(m.a[j]);
+        m.a[j] = norm64r<D>(W + j * D, ok, m.y[j]);
         m.lg[j] = log64(m.a[j]);
 #pragma unroll
         for (int i = 0; i < D; ++i) ok.dividend(W[i + j * D]);

@@ -137,7 +137,8 @@ struct RBenettin {
         if (st.code != 0) return;
         if constexpr (sizeof(T) == 8) {
             Ok ok;
-            const double a = norm64<D>(W, ok), y = rcp64(a), lg = log64(a);
+            double y;
+            const double a = norm64r<D>(W, ok, y), lg = log64(a);
             double u[D];
 #pragma unroll
             for (int l = 0; l < D; ++l) { ok.dividend(W[l]); u[l] = quo64(W[l], a, y); }
@@ -277,8 +278,7 @@ struct RGALI {
             double y[K];
 #pragma unroll
             for (int j = 0; j < K; ++j) {
-                a[j] = norm64<D>(W + j * D, ok);
-                y[j] = rcp64(a[j]);
+                a[j] = norm64r<D>(W + j * D, ok, y[j]);
                 lg[j] = log64(a[j]);
 #pragma unroll
                 for (int i = 0; i < D; ++i) ok.dividend(W[i + j * D]);

@@ -11,6 +11,7 @@
 #include <string>
 
 #include "cl_kernel.cuh"
+#include "cl_pipe.cuh"
 
 namespace cl {
 
@@ -80,10 +81,30 @@ cudaError_t launch_variant(const cl_run& run, const KArgs& a, const double* devA
     return e;
 }
 
-// The compiled variants MB... of one instance; an unknown minb runs the first.
+template <class Sys, class F>
+cudaError_t launch_pipe(const cl_run& run, const KArgs& a, cudaStream_t st, LaunchInfo* info) {
+    const Sys sys = SysMaker<Sys>::make(run, nullptr);
+    auto k = pipe_kernel<Sys, F>;
+    const long long grid = (a.n + 31) / 32;
+    k<<<static_cast<unsigned>(grid), 160, 0, st>>>(a, sys);
+    const cudaError_t e = cudaGetLastError();
+    if (info) {
+        cudaFuncAttributes at;
+        if (cudaFuncGetAttributes(&at, k) == cudaSuccess) info->regs = at.numRegs;
+        info->block = 160;
+        info->grid = static_cast<int>(grid);
+    }
+    return e;
+}
+
+// The compiled variants MB... of one instance; an unknown minb runs the first. Small ensembles of the two-dimensional
+// maps run as a pipeline of warps (cl_pipe.cuh).
 template <class Sys, typename Real, class F0, class F1, class F2, int NF, int... MB>
 cudaError_t launch_instance(const cl_run& run, const KArgs& a, const double* devA, cudaStream_t st, LaunchInfo* info,
                             int minb) {
+    if constexpr (PipeOf<Sys, Real, F0, NF>::ok) {
+        if (a.tau <= PIPE_STEPS && a.n <= PIPE_ORBITS) return launch_pipe<Sys, F0>(run, a, st, info);
+    }
     cudaError_t e = cudaErrorInvalidValue;
     bool done = false;
     ((!done && MB == minb ? (e = launch_variant<Sys, Real, F0, F1, F2, NF, MB>(run, a, devA, st, info), done = true)

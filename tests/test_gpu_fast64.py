@@ -32,7 +32,7 @@ SOURCE = r"""
 #include "cl_fast64.cuh"
 using namespace cl;
 typedef unsigned long long u64;
-__device__ u64 bad[8];
+__device__ u64 bad[9];
 __device__ u64 rnd(u64& s) { s += 0x9e3779b97f4a7c15ULL; return mix64(s); }
 __device__ double mk(u64 r, int e) { return __longlong_as_double((long long)((r & 0xfffffffffffffULL) | ((u64)(1023 + e) << 52))); }
 __device__ bool ne(double a, double b) { return __double_as_longlong(a) != __double_as_longlong(b); }
@@ -56,6 +56,12 @@ __global__ void operands(u64 seed, int iters) {
         if ((a == 0.0 || (fabs(ref) > 1e-290 && fabs(ref) < 1e290)) && ne(quo64(a, b, y), ref)) atomicAdd(&bad[1], 1);
         if (ne(root64(b), sqrt(b))) atomicAdd(&bad[2], 1);
         if (ne(log64(b), cl_log(b)) || ne(log64(c), cl_log(c))) atomicAdd(&bad[3], 1);
+        // a norm with its reciprocal, of two and of four entries
+        Ok okn;
+        const double v[4] = {b, mk(r2, e1 + (int)((r3 >> 33) % 5) - 2), mk(r1 ^ r2, e1 - (int)((r3 >> 36) % 60)), mk(r2 >> 3, e1)};
+        double y2, y4;
+        const double n2 = norm64r<2>(v, okn, y2), n4 = norm64r<4>(v, okn, y4);
+        if (e1 > -600 && e1 < 600 && (!okn.ok || ne(n2, safe_norm<2>(v)) || ne(n4, safe_norm<4>(v)) || ne(y2, 1.0 / n2) || ne(y4, 1.0 / n4))) atomicAdd(&bad[8], 1);
         // quotients nearest a tie: A 2^t - B m = k with m odd, k small
         u64 B = (r1 & 0xfffffffffffffULL) | (1ULL << 52) | 1;
         if (r3 & 1) B |= 0xff00000000000ULL;
@@ -112,11 +118,11 @@ def test_operations_are_the_ieee_ones(tmp_path):
                         "-I" + os.path.join(ROOT, "include"), "-I" + os.path.join(ROOT, "chaos_b200", "csrc"),
                         "-o", str(so), str(src)], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
-    out = (C.c_uint64 * 8)()
+    out = (C.c_uint64 * 9)()
     assert C.CDLL(str(so)).run(out) == 0
-    reciprocal, quotient, root, log, hard_quotient, hard_root, n_quotient, n_root = list(out)
+    reciprocal, quotient, root, log, hard_quotient, hard_root, n_quotient, n_root, norm = list(out)
     assert n_quotient > 1_000_000 and n_root > 10_000
-    assert (reciprocal, quotient, root, log, hard_quotient, hard_root) == (0, 0, 0, 0, 0, 0)
+    assert (reciprocal, quotient, root, log, norm, hard_quotient, hard_root) == (0,) * 7
 
 
 CHAINS = [(2, (QRSpectrum(MGS()),)), (2, (QRSpectrum(CGS()),)), (2, (QRSpectrum(HouseholderQR()),)),
@@ -168,3 +174,22 @@ def test_orbits_that_fail_after_good_handoffs(oracle, k, chain):
         dev, _ = _compare(sysm, x0, 400, fr, 5, oracle, launch_steps=launch)
         assert 0 < np.count_nonzero(dev[0].code) < n
         assert np.any((dev[0].code != 0) & (dev[0].hstep > 10))
+
+
+@pytest.mark.parametrize("chain", [(QRSpectrum(MGS()),), (QRSpectrum(GivensQR()),), (SALI(),), (MEGNO(),),
+                                   (MEGNO(replace=False), FLI(replace=False), SALI())], ids=repr)
+@pytest.mark.parametrize("n,N,tau", [(1, 1, 1), (31, 7, 1), (33, 12, 3), (65, 20, 4), (40, 9, 3), (9473, 10, 2)])
+def test_pipelined_small_ensembles(oracle, n, N, tau, chain):
+    """The pipeline of warps at the edges of its blocks (one step, part of a block, windows that do not fill one, spare
+    lanes), one orbit past its range, and with orbits that stop on the way: huge starts overflow, a frame of zeros and a
+    non-finite one fail at the first handoff, and a kicked map of 1e300 overflows later. Relaunched windows too."""
+    W0 = haar_frames(n, 2, 2, 14)
+    x0 = uniform_starts(n, 2, 15)
+    if n >= 31:
+        W0[3] = 0.0
+        W0[5, 1, 1] = np.inf
+        W0[7] *= 1e250
+        x0[9, 0] = np.nan
+    for K in (6.0, 1e300):
+        for launch in (None, tau):
+            _compare(StandardMap(K), x0, N, [FrameSpec(2, chain, W0)], tau, oracle, launch_steps=launch)
