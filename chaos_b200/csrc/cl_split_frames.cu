@@ -46,6 +46,20 @@ __device__ __forceinline__ void load_stored64(const KArgs& a, int f, i64 i, doub
     for (int l = 0; l < D * K; ++l) W[l] = a.W_out[f][i * so + l * sc];
 }
 
+// The Float32 frame to and from its place in shared memory (8-byte aligned), two entries an access
+__device__ __forceinline__ void park16(float* to, const float* W) {
+#pragma unroll
+    for (int l = 0; l < 8; ++l) reinterpret_cast<float2*>(to)[l] = make_float2(W[2 * l], W[2 * l + 1]);
+}
+__device__ __forceinline__ void unpark16(float* W, const float* from) {
+#pragma unroll
+    for (int l = 0; l < 8; ++l) {
+        const float2 v = reinterpret_cast<const float2*>(from)[l];
+        W[2 * l] = v.x;
+        W[2 * l + 1] = v.y;
+    }
+}
+
 // the Float32 frame holds no non-finite entry (a NaN or infinity turns the fma chain's zero into NaN)
 __device__ __forceinline__ bool finite32(const float* W) {
     float z = 0.0f;
@@ -61,7 +75,7 @@ __device__ __forceinline__ bool finite64(const double* W) {
     return m != 0x7ff00000u;
 }
 __device__ __forceinline__ bool finite_x(const double* x) {
-    return isfin(x[0]) && isfin(x[1]) && isfin(x[2]) && isfin(x[3]);
+    return all_finite_x<4, 4>(x);   // on the integer pipe
 }
 
 // Blocks of 64 threads: 65536 orbits are 1024 blocks, one wave of 148 SMs at 7 blocks per SM. Registers are
@@ -117,6 +131,7 @@ __global__ void __maxnreg__(REGS) split_frames_kernel(const KArgs a, const SysFr
     bool alive0 = code0 == STATUS_OK, alive1 = code1 == STATUS_OK;
     if (!alive0 && !alive1) return;   // frozen since an earlier launch: nothing is rewritten
     const double orth_tol = a.prm[0][0].orthogonality_tol;
+    const bool wide = !a.soa && (reinterpret_cast<uintptr_t>(a.W_out[1]) & 15) == 0;
 
     i64 n = a.n0;
     const i64 handoffs = a.steps / a.tau;
@@ -144,13 +159,14 @@ __global__ void __maxnreg__(REGS) split_frames_kernel(const KArgs a, const SysFr
             int8_t c = xok ? (finite32(W0) ? STATUS_OK : STATUS_W) : STATUS_STATE;
             if (c == STATUS_OK) {
                 // the factorisation runs in the frame's registers: a failing handoff leaves the frame as it was
-#pragma unroll
-                for (int l = 0; l < 16; ++l) park_w[l] = W0[l];
-                split::qr_handoff(q, n, W0, orth_tol);
+                park16(park_w, W0);
+                if (!split::qr_handoff<true>(q, n, W0, orth_tol)) {
+                    unpark16(W0, park_w);
+                    split::qr_handoff<false>(q, n, W0, orth_tol);
+                }
                 if (q.code != 0) {
                     c = STATUS_REDUCER;
-#pragma unroll
-                    for (int l = 0; l < 16; ++l) W0[l] = park_w[l];
+                    unpark16(W0, park_w);
                 }
             }
             if (c != STATUS_OK) { code0 = c; hstep0 = n; alive0 = false; }
@@ -162,17 +178,23 @@ __global__ void __maxnreg__(REGS) split_frames_kernel(const KArgs a, const SysFr
                 // compiler reload them afterwards instead of keeping them in registers)
 #pragma unroll
                 for (int l = 0; l < 4; ++l) park_x[l] = x[l];
-#pragma unroll
-                for (int l = 0; l < 16; ++l) park_w[l] = W0[l];
+                park16(park_w, W0);
                 asm volatile("" ::: "memory");
                 // the unit columns of a successful handoff go to the frame's output, where the values are formed
                 // from them once, after the loop (the last successful handoff's are the ones the state keeps)
-                if (split::gali_step(g, n, W1)) store_frame(a, 1, i, W1);
+                if (split::gali_step(g, n, W1)) {
+                    if (wide) {   // a column's halves in one store each
+                        double2* o = reinterpret_cast<double2*>(a.W_out[1] + i * D * K);
+#pragma unroll
+                        for (int l = 0; l < 8; ++l) o[l] = make_double2(W1[2 * l], W1[2 * l + 1]);
+                    } else {
+                        store_frame(a, 1, i, W1);
+                    }
+                }
                 asm volatile("" ::: "memory");
 #pragma unroll
                 for (int l = 0; l < 4; ++l) x[l] = park_x[l];
-#pragma unroll
-                for (int l = 0; l < 16; ++l) W0[l] = park_w[l];
+                unpark16(W0, park_w);
                 if (g.gcode != 0 || g.scode != 0) c = STATUS_REDUCER;
             }
             if (c != STATUS_OK) { code1 = c; hstep1 = n; alive1 = false; }

@@ -176,10 +176,36 @@ struct QRSlot {
     int code, pad;
 };
 
+// Float32 reciprocal and square root without a branch, for operands with an exponent within +-100: the hardware estimate
+// and one residual correction give the IEEE result for every significand (checked over all of them,
+// tests/test_gpu_fast64.py), where `/` and sqrtf() carry a branch to a general routine each.
+__device__ __forceinline__ float rcp32(float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
+}
+__device__ __forceinline__ float root32(float s) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
+    const float g = s * y;
+    return __fmaf_rn(__fmaf_rn(-g, g, s), 0.5f * y, g);
+}
+__device__ __forceinline__ bool mid32(float v) {   // positive, exponent within +-60
+    return __float_as_uint(v) - ((127u - 60u) << 23) < (120u << 23);
+}
+
 // One handoff (qr_spectrum.jl:50-73 with householder.jl:19-80): W (4 x 4, column-major) is replaced by Q. The
 // factorisation runs in W's own registers (A aliases W; its lower part is dead once the reflectors are taken, its
 // upper part is R), so the handoff needs only the reflectors and R's inverse besides the frame.
-__device__ __forceinline__ void qr_handoff(QRSlot& st, i64 n, float* W, double orth_tol) {
+// FAST: with the branch-free reciprocals and roots; returns false, with the slot untouched and W spent, when an operand
+// leaves their range or a check fails (the caller restores W and takes the general form). The handoff has 7 reciprocals
+// and 5 roots; with the indicator frame's checks on the exponents too, 65536 orbits x 4000 steps 3.80 -> 3.54 ms, 4096
+// orbits 2.46 -> 2.09.
+template <bool FAST>
+__device__ __forceinline__ bool qr_handoff(QRSlot& st, i64 n, float* W, double orth_tol) {
+    auto rcp = [](float b) { return FAST ? rcp32(b) : 1.0f / b; };
+    auto root = [](float v) { return FAST ? root32(v) : sqrtf(v); };
+    bool in = true;
     float* A = W;
     float V[10], beta[3];   // reflector j: rows j..3 at V[off_j..], off = 0, 4, 7
     int count = 0;
@@ -190,18 +216,19 @@ __device__ __forceinline__ void qr_handoff(QRSlot& st, i64 n, float* W, double o
         float s2 = A[j + 4 * j] * A[j + 4 * j];
 #pragma unroll
         for (int i = j + 1; i < 4; ++i) s2 = __fmaf_rn(A[i + 4 * j], A[i + 4 * j], s2);
-        const float c = sqrtf(s2);
+        in = in && mid32(s2);
+        const float c = root(s2);
         float rho = c;
         beta[j] = 0.0f;
 #pragma unroll
         for (int i = j; i < 4; ++i) V[off + i - j] = 0.0f;
-        if (isfin(c) && c > 0.0f) {
+        if (FAST || (isfin(c) && c > 0.0f)) {
             const float ajj = A[j + 4 * j];
             const float sg = ajj < 0.0f ? -1.0f : 1.0f;
             V[off] = ajj + sg * c;
 #pragma unroll
             for (int i = j + 1; i < 4; ++i) V[off + i - j] = A[i + 4 * j];
-            beta[j] = 1.0f / (c * (c + fabsf(ajj)));   // 2 / |v|^2
+            beta[j] = rcp(c * (c + fabsf(ajj)));   // 2 / |v|^2
             // the columns right of the pivot, rows j..3: A_l -= beta (v . A_l) v
 #pragma unroll
             for (int l = j + 1; l < 4; ++l) {
@@ -225,22 +252,27 @@ __device__ __forceinline__ void qr_handoff(QRSlot& st, i64 n, float* W, double o
     for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int i = 0; i <= j; ++i) A[i + 4 * j] *= sg[i];
+    if (FAST) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) in = in && mid32(A[j + 4 * j]);
+        if (!in) return false;
+    }
     int bad = 0;   // _factor_failure (qr_spectrum.jl:43-48): the first pivot that is not finite and positive
 #pragma unroll
     for (int j = 3; j >= 0; --j)
-        if (!(isfin(A[j + 4 * j]) && A[j + 4 * j] > 0.0f)) bad = j + 1;
+        if (!FAST && !(isfin(A[j + 4 * j]) && A[j + 4 * j] > 0.0f)) bad = j + 1;
     if (bad) {
         float pv = A[0];
 #pragma unroll
         for (int j = 0; j < 4; ++j) if (j + 1 == bad) pv = A[j + 4 * j];
         st.code = 1; st.column = bad; st.value = pv; st.threshold = isfin(pv) ? 0.0 : __longlong_as_double(0x7ff0000000000000LL);
         st.step = n;
-        return;
+        return true;
     }
     // window_Gw (orthonormalize.jl:112-127): |R|_F |R^-1|_F, R^-1 by back substitution with the pivots' reciprocals
     float rd[4], rin[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { rd[i] = A[i + 4 * i]; rin[i] = 1.0f / rd[i]; }
+    for (int i = 0; i < 4; ++i) { rd[i] = A[i + 4 * i]; rin[i] = rcp(rd[i]); }
     float ra = 0.0f, rb = 0.0f;
     {
         float Ri[16];
@@ -260,7 +292,8 @@ __device__ __forceinline__ void qr_handoff(QRSlot& st, i64 n, float* W, double o
 #pragma unroll
             for (int i = 0; i <= j; ++i) { ra = __fmaf_rn(A[i + 4 * j], A[i + 4 * j], ra); rb = __fmaf_rn(Ri[i + 4 * j], Ri[i + 4 * j], rb); }
     }
-    const float Gw = sqrtf(ra) * sqrtf(rb);
+    if (FAST && !(mid32(ra) && mid32(rb))) return false;
+    const float Gw = root(ra) * root(rb);
     // Q = H_0 H_1 H_2 I, formed in W's registers (R is no longer needed but its diagonal, kept in rd): each H_j
     // touches rows j..3 of the columns j..3 (the columns left of j are still e_l there); then the column signs
     float* Q = W;
@@ -298,16 +331,19 @@ __device__ __forceinline__ void qr_handoff(QRSlot& st, i64 n, float* W, double o
         }
     const float thr = static_cast<float>(orth_tol) * 0x1p-23f * 4.0f;   // tol eps(Float32) k g, g = 1 (Householder)
     if (!(orth <= thr)) {
+        if (FAST) return false;
         st.code = 4; st.column = 0; st.value = orth; st.threshold = thr; st.step = n;
-        return;
+        return true;
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) lp_mul(st.lp[i], static_cast<double>(rd[i]));
     st.n = n;
-    st.G_max = jl_max(st.G_max, static_cast<double>(Gw));   // _G_from_Gw is G_w for k > 2
-    st.orth_max = jl_max(st.orth_max, static_cast<double>(orth));
+    const double G = static_cast<double>(Gw), O = static_cast<double>(orth);   // _G_from_Gw is G_w for k > 2
+    st.G_max = FAST ? (G > st.G_max ? G : st.G_max) : jl_max(st.G_max, G);
+    st.orth_max = FAST ? (O > st.orth_max ? O : st.orth_max) : jl_max(st.orth_max, O);
     st.count_max = st.count_max > count ? st.count_max : count;
     st.column = 0;
+    return true;
 }
 
 // ---- the indicator frame: GALI_4 with SALI of its columns 1-2, Float64 ------------------------------------------
@@ -330,6 +366,26 @@ __device__ __forceinline__ bool gali_step(GSSlot& st, i64 n, double* W) {
     double s[4], a[4], inv[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) s[j] = sumsq64<4>(W + 4 * j);
+    // every sum of squares normal (the exponent field neither 0 nor all ones): then every norm is finite, positive and
+    // above the smallest normal, and both reducers' checks hold
+    bool normal = st.scode == 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) normal = normal && static_cast<unsigned>(__double2hiint(s[j])) - 0x00100000u < 0x7fe00000u;
+    if (normal) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            inv[j] = rsq64(s[j]);
+            lp_mul(st.lp[j], s[j] * inv[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) W[i + 4 * j] *= inv[j];
+        st.sn = n;
+        st.gn = n;
+        st.pending = 3;
+        return true;
+    }
     const double fm = 2.2250738585072014e-308;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

@@ -30,9 +30,10 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SOURCE = r"""
 #include "chaoslab_b200.h"
 #include "cl_fast64.cuh"
+#include "cl_split_frames.cuh"
 using namespace cl;
 typedef unsigned long long u64;
-__device__ u64 bad[9];
+__device__ u64 bad[11];
 __device__ u64 rnd(u64& s) { s += 0x9e3779b97f4a7c15ULL; return mix64(s); }
 __device__ double mk(u64 r, int e) { return __longlong_as_double((long long)((r & 0xfffffffffffffULL) | ((u64)(1023 + e) << 52))); }
 __device__ bool ne(double a, double b) { return __double_as_longlong(a) != __double_as_longlong(b); }
@@ -100,9 +101,20 @@ __global__ void roots() {
         }
     }
 }
+// the Float32 reciprocal and root of the split kernel, every significand, at the ends and the middle of their range
+__global__ void all32() {
+    const unsigned m = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int e = -100; e <= 100; e += 50)
+        for (int odd = 0; odd < 2; ++odd) {
+            const float v = __uint_as_float(m | static_cast<unsigned>(127 + e + odd) << 23);
+            if (__float_as_uint(split::rcp32(v)) != __float_as_uint(1.0f / v)) atomicAdd(&bad[9], 1);
+            if (__float_as_uint(split::root32(v)) != __float_as_uint(sqrtf(v))) atomicAdd(&bad[10], 1);
+        }
+}
 extern "C" int run(unsigned long long* out) {
     operands<<<148 * 8, 256>>>(1, 400);
     roots<<<32, 256>>>();
+    all32<<<(1 << 23) / 256, 256>>>();
     if (cudaDeviceSynchronize() != cudaSuccess) return 1;
     return cudaMemcpyFromSymbol(out, bad, sizeof bad) == cudaSuccess ? 0 : 2;
 }
@@ -118,11 +130,11 @@ def test_operations_are_the_ieee_ones(tmp_path):
                         "-I" + os.path.join(ROOT, "include"), "-I" + os.path.join(ROOT, "chaos_b200", "csrc"),
                         "-o", str(so), str(src)], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
-    out = (C.c_uint64 * 9)()
+    out = (C.c_uint64 * 11)()
     assert C.CDLL(str(so)).run(out) == 0
-    reciprocal, quotient, root, log, hard_quotient, hard_root, n_quotient, n_root, norm = list(out)
+    reciprocal, quotient, root, log, hard_quotient, hard_root, n_quotient, n_root, norm, rcp32, root32 = list(out)
     assert n_quotient > 1_000_000 and n_root > 10_000
-    assert (reciprocal, quotient, root, log, norm, hard_quotient, hard_root) == (0,) * 7
+    assert (reciprocal, quotient, root, log, norm, hard_quotient, hard_root, rcp32, root32) == (0,) * 9
 
 
 CHAINS = [(2, (QRSpectrum(MGS()),)), (2, (QRSpectrum(CGS()),)), (2, (QRSpectrum(HouseholderQR()),)),
