@@ -1257,8 +1257,9 @@ int64_t cl_b200_mlp_train_workspace(int32_t B) {
 int cl_b200_mlp_train_step(const void* X, int32_t B, const void* const* layers, const float* label, const float* target,
                            float w_reg, float lr, float b1, float b2, float eps, int32_t t, void* workspace,
                            int64_t workspace_bytes, float* row_loss, void* stream) {
-    if (!X || !layers || !label || !target || !workspace || !row_loss || B <= 0 || B % BM || t < 1)
-        return capi_fail(CL_EINVAL, "train step: bad arguments (a batch is a positive multiple of 128 rows)");
+    // the transpose's grid has a block per 32 rows in y
+    if (!X || !layers || !label || !target || !workspace || !row_loss || B <= 0 || B % BM || B > 32 * 65535 || t < 1)
+        return capi_fail(CL_EINVAL, "train step: bad arguments (a batch is a positive multiple of 128 rows, at most 2097120)");
     for (int i = 0; i < 10 * T_LAYERS; ++i)
         if (!layers[i] || reinterpret_cast<uintptr_t>(layers[i]) % 16)
             return capi_fail(CL_EINVAL, "train step: every layer array needs 16-byte alignment");

@@ -3,8 +3,9 @@ kernels (`cl_b200_gemm_bf16`: tcgen05.mma with a tensor-memory accumulator) and 
 
 64 inputs -> 256 -> 256 -> 256 (GELU, tanh form) -> 2 outputs: the logit of P(chaotic) and a prediction of the
 final lambda_1. Inference runs the whole network in one persistent tensor-core kernel (`cl_b200_mlp_forward_fused`)
-on weights packed once into the MMA layout; training runs it layer by layer, keeping the pre-activations. No reference counterpart: the reference has no learned component. PyTorch only holds the device buffers
-and the stream; every arithmetic step runs in the library's kernels.
+on weights packed once into the MMA layout; a training step is one native call of ten launches
+(`cl_b200_mlp_train_step`). No reference counterpart: the reference has no learned component. PyTorch only holds the
+device buffers and the stream; every arithmetic step runs in the library's kernels.
 
 Training is mean binary cross-entropy on the label plus `w_reg` times the mean squared error on lambda_1, with Adam
 on FP32 master weights whose BF16 copies (and their transposes, for the backward GEMMs) feed the tensor cores.
@@ -12,7 +13,9 @@ on FP32 master weights whose BF16 copies (and their transposes, for the backward
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
+import operator
 
 import numpy as np
 
@@ -20,6 +23,7 @@ from ._lib import last_error, lib
 
 DIMS = (64, 256, 256, 256, 2)
 OUT_PAD = 16   # the last layer's 2 outputs padded to the smallest tensor-core N tile
+TRAIN_ROWS = 32 * 65535   # the most rows a training step's transposes take (a block per 32 rows in a grid's y)
 
 
 def _ck(rc, what):
@@ -245,21 +249,24 @@ class MLP:
 
     def train_step(self, Xb, label, target, w_reg=1.0, lr=1e-3):
         """Forward, loss, gradients (in each layer's gW, gb) and Adam on one batch; returns the row losses. Batches of
-        whole 128-row tiles run as one native call (ten launches); others pass by pass."""
-        B = Xb.shape[0]
-        if self.dims == DIMS and B % 128 == 0 and B:
+        whole 128-row tiles of 64 features run as one native call (ten launches); others (wider rows, of which the
+        first 64 columns count, arrays off 16 bytes, a subclass's own passes) pass by pass."""
+        B, native = Xb.shape[0], type(self) is MLP and self.dims == DIMS and Xb.shape[1] == DIMS[0]
+        if native and 0 < B <= TRAIN_ROWS and B % 128 == 0 and self.step >= 0:
             t, L = self.t, _declare(lib())
-            Xb, label, target = Xb.contiguous(), label.contiguous(), target.contiguous()
-            nbytes = L.cl_b200_mlp_train_workspace(B)
-            ws = t.empty(nbytes, dtype=t.uint8, device=self.dev)
-            rl = t.empty(B, dtype=t.float32, device=self.dev)
-            ptrs = (C.c_void_p * 40)(*[lay[k].data_ptr() for lay in self.layers
-                                       for k in ("W", "b", "Wb", "Wbt", "mW", "vW", "mb", "vb", "gW", "gb")])
-            _ck(L.cl_b200_mlp_train_step(Xb.data_ptr(), B, ptrs, label.data_ptr(), target.data_ptr(), w_reg, lr, 0.9,
-                                         0.999, 1e-8, self.step + 1, ws.data_ptr(), nbytes, rl.data_ptr(),
-                                         self.stream()), "train step")
-            self.step += 1
-            return rl
+            X = Xb.contiguous()
+            ptrs = [lay[k].data_ptr() for lay in self.layers
+                    for k in ("W", "b", "Wb", "Wbt", "mW", "vW", "mb", "vb", "gW", "gb")]
+            if not functools.reduce(operator.or_, ptrs, X.data_ptr()) % 16:
+                label, target = label.contiguous(), target.contiguous()
+                nbytes = L.cl_b200_mlp_train_workspace(B)
+                ws = t.empty(nbytes, dtype=t.uint8, device=self.dev)
+                rl = t.empty(B, dtype=t.float32, device=self.dev)
+                _ck(L.cl_b200_mlp_train_step(X.data_ptr(), B, (C.c_void_p * 40)(*ptrs), label.data_ptr(),
+                                             target.data_ptr(), w_reg, lr, 0.9, 0.999, 1e-8, self.step + 1,
+                                             ws.data_ptr(), nbytes, rl.data_ptr(), self.stream()), "train step")
+                self.step += 1
+                return rl
         out = self.forward(Xb, keep=True)
         rl, g32, gb = self.loss_and_grad(out, label, target, w_reg)
         self.backward(g32, gb)

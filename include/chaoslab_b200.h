@@ -461,7 +461,7 @@ CL_API int cl_b200_mlp_forward_fused(const void* X, int32_t B, const void* Wp1, 
 /* 0, or CL_EDEVICE_LOST after a bounded wait on an MMA or copy barrier (GEMM or fused pass) gave up. */
 CL_API int cl_b200_mlp_status(void);
 /* One training step of that network: forward, mean binary cross-entropy on `label` plus w_reg times the mean squared
- * error on `target`, gradients, Adam (step count t), with the row losses in row_loss. B is a multiple of 128; `layers`
+ * error on `target`, gradients, Adam (step count t), with the row losses in row_loss. B is a multiple of 128, at most 2097120; `layers`
  * holds, for each of the four layers in order, the device pointers {W, b, W in BF16, its transpose in BF16, Adam's m and
  * v of W, m and v of b, the gradients of W and b} (FP32 but the BF16 copies; the last layer's 2 outputs padded to 16).
  * `workspace`: cl_b200_mlp_train_workspace(B) bytes, 256-byte aligned, free again when the stream has passed the call. */

@@ -65,3 +65,35 @@ def test_step_equals_the_passes(rows):
         for key in ("W", "b", "mW", "vW", "mb", "vb", "Wb", "Wbt"):
             assert torch.equal(lay[key], lb[key]), key
     assert a.step == b.step == 101
+
+
+class _Own(MLP):
+    def adam(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
+        super().adam(lr=0.0, b1=b1, b2=b2, eps=eps)
+
+
+# what the native step does not take runs pass by pass, with those passes' result
+@pytest.mark.parametrize("form", ["wide", "ragged", "bias off 16 bytes", "subclass"])
+def test_other_calls_take_the_passes(form):
+    import torch
+    dev = torch.device("cuda", 0)
+    rng = np.random.default_rng(11)
+    rows, cols = 200 if form == "ragged" else 256, 72 if form == "wide" else 64
+    X = torch.tensor(rng.standard_normal((rows, cols)).astype(np.float32), device=dev).to(torch.bfloat16)
+    label = torch.tensor((rng.random(rows) < 0.5).astype(np.float32), device=dev)
+    target = torch.tensor(rng.standard_normal(rows).astype(np.float32), device=dev)
+    a, b = _net(torch, dev), _net(torch, dev)
+    if form == "subclass":
+        a.__class__ = b.__class__ = _Own
+    if form == "bias off 16 bytes":
+        for n in (a, b):
+            n.layers[1]["b"] = torch.cat([n.layers[1]["b"][:1], n.layers[1]["b"]])[1:]
+    loss = a.train_step(X, label, target, w_reg=0.7, lr=2e-3)
+    out = b.forward(X, keep=True)
+    loss_b, g32, gb = b.loss_and_grad(out, label, target, 0.7)
+    b.backward(g32, gb)
+    b.adam(lr=2e-3)
+    assert torch.equal(loss, loss_b) and a.step == b.step == 101
+    for lay, lb in zip(a.layers, b.layers):
+        for key in ("W", "b", "mW", "vW", "mb", "vb", "Wb", "Wbt"):   # one partial sum at these sizes: bit for bit
+            assert torch.equal(lay[key], lb[key]), key
