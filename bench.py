@@ -62,8 +62,8 @@ NU = KAPPA = 1.5
 MU = 0.05
 SEED = 1
 # DRAM bytes per orbit of one launch of the mixed kernel: ncu DRAM read + write of split_frames_kernel on 65536
-# orbits x 2000 steps (15.53 MB read, 1.48 MB written: the orbit, both frames and the records once in, once out)
-TRAFFIC_PER_ORBIT = 17013504 / 65536
+# orbits x 2000 steps (16.01 MB read, 1.89 MB written: the orbit, both frames and the records once in, once out)
+TRAFFIC_PER_ORBIT = 17899008 / 65536
 METRIC = "orbit-steps/s (4D coupled standard maps, QRSpectrum(Householder) + GALI_4 + SALI, mixed-precision kernel)"
 # the headline kernel: Float64 orbit and GALI / SALI frame, Float32 QRSpectrum frame (the precision every output holds)
 HEADLINE = "mixed-ind64"
@@ -82,8 +82,7 @@ HEADLINE = "mixed-ind64"
 #   the stop and carry the frame); k + k logs with a Neumaier add (4 flops) each: 32 (Float64 in both kernels)
 #   once per run: GALI's values, the twice-orthogonalised Gram-Schmidt 2 sum_j j 4 d = 192, the nested norms 2 d k
 #   and scaling d k, the k - 1 products, and SALI 3 d 2 = 24: 267. A handoff's values are overwritten by the next
-#   one and read only after the last (gali.jl:156, sali.jl:108), so the algorithm needs them once; the mixed kernel
-#   forms them once a launch, the Float64 kernel (the reference's loop, bit for bit) at every handoff
+#   one and read only after the last (gali.jl:156, sali.jl:108), so they are needed, and formed, once a launch
 def flops_per_orbit_step(tau: int = TAU, precision: str = "fp64", n_steps: int = N_STEPS) -> dict:
     d, k = 4, 4
     map_flops, trig = 20, 6
@@ -418,12 +417,12 @@ def main() -> None:
             roofline=dict(bound="fp64", achieved=achieved, peak=fp64_peak, unit="TFLOP/s", frac=achieved / fp64_peak,
                           traffic=TRAFFIC_PER_ORBIT * n,
                           traffic_source="ncu dram__bytes_read + dram__bytes_write of split_frames_kernel on 65536 "
-                                         "orbits x 2000 steps (1.701e7 B), scaled by orbits: DRAM bytes grow with the "
+                                         "orbits x 2000 steps (1.790e7 B), scaled by orbits: DRAM bytes grow with the "
                                          "orbits loaded and stored, not with the steps",
                           peak_source="cuBLAS DGEMM 8192^3 measured here (burst)",
                           flops_per_orbit_step=fl,
-                          pipes_ncu=dict(fp64=0.448, fma_fp32=0.140, alu=0.234, xu_sfu=0.171, issue_active=0.632,
-                                         warps_active=0.171,
+                          pipes_ncu=dict(fp64=0.468, fma_fp32=0.143, alu=0.209, xu_sfu=0.181, issue_active=0.622,
+                                         warps_active=0.164,
                                          source="ncu --set full of split_frames_kernel, 65536 orbits x 2000 steps "
                                                 "(profiles/split_frames_kernel_froeschle_65536x2000_ncu.md)")),
             cpu_baseline=cpu, clocks=clocks, gpu_launches=int(launches),
