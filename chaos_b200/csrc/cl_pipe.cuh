@@ -134,20 +134,95 @@ struct PipeWords {
     }
 };
 
+// What the warps hand on, and the parts of warps 0 to 3 for one block of steps. JACS: the tangent entries at the handoffs'
+// points go along with them (the recorder's monitor).
+template <int D, int S, int K, int MN, bool JACS>
+struct PipeShared {
+    static constexpr int B = PIPE_STEPS;
+    double sc[2][B][32];             // the tangent entry of each step: warp 0 -> 1
+    double sx[4][B][S][32];          // the point at each handoff: warp 0 -> 4, three blocks later
+    double sw[3][B][D * K][32];      // the arriving frame at each handoff: warp 1 -> 2, 3 and 4
+    double sm[2][B][MN][32];         // its measures: warps 2, 3 -> 4
+    double sj[JACS ? 4 : 1][JACS ? B : 1][JACS ? 32 : 1];   // the tangent entry at each handoff's point: warp 0 -> 4
+    int sok[2][B][32];
+    int running;
+};
+
+template <class Sys, class R, class M, int K, bool JACS>
+struct PipeParts {
+    static constexpr int D = Sys::D, S = Sys::S;
+    using MW = PipeWords<M, D, K>;
+    using Shared = PipeShared<D, S, K, MW::n, JACS>;
+    // warp 0: the points of block p
+    static __device__ __forceinline__ void points(Shared& sh, const Sys& sys, double* x, StdJac& J, i64 p, int hs, int tau, int lane) {
+        int t = 0;
+        for (int h = 0; h < hs; ++h) {
+            for (int q = 0; q < tau; ++q, ++t) {
+                sh.sc[p & 1][t][lane] = J.c;
+                sys.forward(x, J);
+                sys.jac(x, J);
+            }
+#pragma unroll
+            for (int q = 0; q < S; ++q) sh.sx[p & 3][h][q][lane] = x[q];
+            if constexpr (JACS) sh.sj[p & 3][h][lane] = J.c;
+        }
+    }
+    // warp 1: the frames of block b
+    static __device__ __forceinline__ void frames(Shared& sh, const Sys& sys, double* W, double tol, i64 b, int hs, int tau, int lane) {
+        int t = 0;
+        for (int h = 0; h < hs; ++h) {
+            for (int q = 0; q < tau; ++q, ++t) {
+                StdJac Jt;
+                Jt.s = 0.0;
+                Jt.c = sh.sc[b & 1][t][lane];
+                sys.template apply<K>(Jt, W);
+            }
+#pragma unroll
+            for (int l = 0; l < D * K; ++l) sh.sw[b % 3][h][l][lane] = W[l];
+            pipe_next<R, D, K>(W, tol);
+        }
+    }
+    // warps 2 and 3: the measures of block b's handoffs h0 and h0 + 2
+    static __device__ __forceinline__ void measures(Shared& sh, const RedParams* prm, i64 b, int hs, int h0, int lane) {
+        auto take = [&](int h, M& m) {
+            double W[D * K];
+#pragma unroll
+            for (int l = 0; l < D * K; ++l) W[l] = sh.sw[b % 3][h][l][lane];
+            m.take(W, prm);
+        };
+        auto put = [&](int h, const M& m) {
+            sh.sok[b & 1][h][lane] = MW::put(m, [&](int l, double v) { sh.sm[b & 1][h][l][lane] = v; });
+        };
+        M m0, m1;
+        if (h0 + 2 < hs) {   // both of this warp's handoffs side by side
+            take(h0, m0);
+            take(h0 + 2, m1);
+            put(h0, m0);
+            put(h0 + 2, m1);
+        } else if (h0 < hs) {
+            take(h0, m0);
+            put(h0, m0);
+        }
+    }
+    // warp 4: what arrives at handoff h of block b
+    static __device__ __forceinline__ void arrive(const Shared& sh, double* W, double* x, M& m, i64 b, int h, int lane) {
+#pragma unroll
+        for (int l = 0; l < D * K; ++l) W[l] = sh.sw[b % 3][h][l][lane];
+#pragma unroll
+        for (int q = 0; q < S; ++q) x[q] = sh.sx[b & 3][h][q][lane];
+        MW::get(m, sh.sok[b & 1][h][lane] != 0, [&](int l) { return sh.sm[b & 1][h][l][lane]; });
+    }
+};
+
 template <class Sys, class F>
 __global__ void __launch_bounds__(160, 2) pipe_kernel(const KArgs a, const Sys sys) {
     constexpr int D = Sys::D, S = Sys::S, K = F::K, B = PIPE_STEPS;
     using R = typename PipeFrame<F>::R;
     using M = typename F::template Measure_<D, double>;
-    using MW = PipeWords<M, D, K>;
+    using P = PipeParts<Sys, R, M, K, false>;
     static_assert(M::qr != M::pair, "one kind of measure");
     constexpr bool DEFER = F::defers;
-    __shared__ double sc[2][B][32];             // the tangent entry of each step: warp 0 -> 1
-    __shared__ double sx[4][B][S][32];          // the point at each handoff: warp 0 -> 4, three blocks later
-    __shared__ double sw[3][B][D * K][32];      // the arriving frame at each handoff: warp 1 -> 2, 3 and 4
-    __shared__ double sm[2][B][MW::n][32];      // its measures: warps 2, 3 -> 4
-    __shared__ int sok[2][B][32];
-    __shared__ int running;
+    __shared__ typename P::Shared sh;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const i64 orbit = static_cast<i64>(blockIdx.x) * 32 + lane;
     const bool mine = orbit < a.n;
@@ -169,66 +244,20 @@ __global__ void __launch_bounds__(160, 2) pipe_kernel(const KArgs a, const Sys s
     const bool was = warp == 4 && mine && (fresh || fr.alive);   // not frozen since an earlier launch
     Kept<DEFER, D * K, double> kept;
     if (warp == 0) sys.jac(x, J);
-    if (threadIdx.x == 0) running = 1;
+    if (threadIdx.x == 0) sh.running = 1;
     i64 n = a.n0;
     __syncthreads();
 
     for (i64 p = 0; p < blocks + 3; ++p) {
         if (warp == 0) {
-            if (p < blocks) {
-                const int hs = in_block(p);
-                int t = 0;
-                for (int h = 0; h < hs; ++h) {
-                    for (int q = 0; q < a.tau; ++q, ++t) {
-                        sc[p & 1][t][lane] = J.c;
-                        sys.forward(x, J);
-                        sys.jac(x, J);
-                    }
-#pragma unroll
-                    for (int q = 0; q < S; ++q) sx[p & 3][h][q][lane] = x[q];
-                }
-            }
+            if (p < blocks) P::points(sh, sys, x, J, p, in_block(p), a.tau, lane);
         } else if (warp == 1) {
             const i64 b = p - 1;
-            if (b >= 0 && b < blocks) {
-                const int hs = in_block(b);
-                int t = 0;
-                for (int h = 0; h < hs; ++h) {
-                    for (int q = 0; q < a.tau; ++q, ++t) {
-                        StdJac Jt;
-                        Jt.s = 0.0;
-                        Jt.c = sc[b & 1][t][lane];
-                        sys.template apply<K>(Jt, fr.W);
-                    }
-#pragma unroll
-                    for (int l = 0; l < D * K; ++l) sw[b % 3][h][l][lane] = fr.W[l];
-                    pipe_next<R, D, K>(fr.W, a.prm[0][PipeFrame<F>::at].orthogonality_tol);
-                }
-            }
+            if (b >= 0 && b < blocks)
+                P::frames(sh, sys, fr.W, a.prm[0][PipeFrame<F>::at].orthogonality_tol, b, in_block(b), a.tau, lane);
         } else if (warp < 4) {
             const i64 b = p - 2;
-            if (b >= 0 && b < blocks) {
-                const int hs = in_block(b), h0 = warp - 2;
-                auto take = [&](int h, M& m) {
-                    double W[D * K];
-#pragma unroll
-                    for (int l = 0; l < D * K; ++l) W[l] = sw[b % 3][h][l][lane];
-                    m.take(W, a.prm[0]);
-                };
-                auto put = [&](int h, const M& m) {
-                    sok[b & 1][h][lane] = MW::put(m, [&](int l, double v) { sm[b & 1][h][l][lane] = v; });
-                };
-                M m0, m1;
-                if (h0 + 2 < hs) {   // both of this warp's handoffs side by side
-                    take(h0, m0);
-                    take(h0 + 2, m1);
-                    put(h0, m0);
-                    put(h0 + 2, m1);
-                } else if (h0 < hs) {
-                    take(h0, m0);
-                    put(h0, m0);
-                }
-            }
+            if (b >= 0 && b < blocks) P::measures(sh, a.prm[0], b, in_block(b), warp - 2, lane);
         } else {
             const i64 b = p - 3;
             if (b >= 0) {
@@ -237,20 +266,16 @@ __global__ void __launch_bounds__(160, 2) pipe_kernel(const KArgs a, const Sys s
                     n += a.tau;
                     if (!fr.alive) continue;
                     kept.take(fr.W);
-#pragma unroll
-                    for (int l = 0; l < D * K; ++l) fr.W[l] = sw[b % 3][h][l][lane];
-#pragma unroll
-                    for (int q = 0; q < S; ++q) x[q] = sx[b & 3][h][q][lane];
                     M m;
-                    MW::get(m, sok[b & 1][h][lane] != 0, [&](int l) { return sm[b & 1][h][l][lane]; });
+                    P::arrive(sh, fr.W, x, m, b, h, lane);
                     frame_handoff<D, S, DEFER>(fr, x, n, a.prm[0], m);
                 }
                 const bool any = __any_sync(0xffffffffu, fr.alive);
-                if (lane == 0) running = any;
+                if (lane == 0) sh.running = any;
             }
         }
         __syncthreads();
-        if (!running) break;
+        if (!sh.running) break;
         __syncthreads();   // `running` is read before the next block may write it
     }
     if (!was) return;

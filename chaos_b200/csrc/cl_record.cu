@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -103,6 +104,28 @@ template <int ALG> struct EstFinal<RQR<ALG>> {
     }
 };
 
+// _dev_row! (run_device.jl:10-22): row g of an orbit's record
+template <int S, int K>
+__device__ __forceinline__ void record_row(double* Ri, int g, const double* lam, double orth, double gmax,
+                                           const MonState& mon, const double* x) {
+    constexpr int NCOL = K + 7 + S;
+    double* row = Ri + static_cast<i64>(g) * NCOL;
+#pragma unroll
+    for (int j = 0; j < K; ++j) row[j] = lam[j];
+    row[K] = mon.det_max;
+    row[K + 1] = mon.symp_max;
+    row[K + 2] = orth;
+    if constexpr (K == 2) {   // _dev_sumpair!: eps_sum = |l1 + l2|, eps_pair = max_i |l_i + l_(3-i)| = |l1 + l2|
+        const double sp = fabs(lam[0] + lam[1]);
+        row[K + 3] = g > 0 ? jl_max(row[K + 3 - NCOL], sp) : sp;
+        row[K + 4] = g > 0 ? jl_max(row[K + 4 - NCOL], sp) : sp;
+    }
+    row[K + 5] = gmax;
+    row[K + 6] = mon.M_max;
+#pragma unroll
+    for (int j = 0; j < S; ++j) row[K + 7 + j] = x[j];
+}
+
 template <class Sys, class Est, int K, typename Real>
 __global__ void __launch_bounds__(128) record_kernel(const RecArgs a, const Sys sys) {
     using O = RecOrbit<Sys, Est, K, Real>;
@@ -137,24 +160,9 @@ __global__ void __launch_bounds__(128) record_kernel(const RecArgs a, const Sys 
         c = o.body(sys, n, target - n, a.N, a.tau, a.prm);
         h = n;
         if (c != STATUS_OK) { a.fail[i] = g + 1; break; }
-        // _dev_row! (run_device.jl:10-22)
         double lam[K], orth, gmax;
         EstFinal<Est>::get(o.est.head, lam, orth, gmax);
-        double* row = Ri + static_cast<i64>(g) * NCOL;
-#pragma unroll
-        for (int j = 0; j < K; ++j) row[j] = lam[j];
-        row[K] = o.mon.det_max;
-        row[K + 1] = o.mon.symp_max;
-        row[K + 2] = orth;
-        if constexpr (K == 2) {   // _dev_sumpair!: eps_sum = |l1 + l2|, eps_pair = max_i |l_i + l_(3-i)| = |l1 + l2|
-            const double sp = fabs(lam[0] + lam[1]);
-            row[K + 3] = g > 0 ? jl_max(row[K + 3 - NCOL], sp) : sp;
-            row[K + 4] = g > 0 ? jl_max(row[K + 4 - NCOL], sp) : sp;
-        }
-        row[K + 5] = gmax;
-        row[K + 6] = o.mon.M_max;
-#pragma unroll
-        for (int j = 0; j < S; ++j) row[K + 7 + j] = o.x[j];
+        record_row<S, K>(Ri, g, lam, orth, gmax, o.mon, o.x);
     }
     if (c == STATUS_OK && n < a.n0 + a.steps) {
         c = o.body(sys, n, a.n0 + a.steps - n, a.N, a.tau, a.prm);
@@ -173,11 +181,143 @@ __global__ void __launch_bounds__(128) record_kernel(const RecArgs a, const Sys 
     if (a.hstep) a.hstep[i] = h;
 }
 
+// The same for small Float64 ensembles as a pipeline of five warps per 32 orbits (cl_pipe.cuh): warp 4 takes the
+// estimator's sums, the monitor (on the tangent entries warp 0 has at the handoffs) and the rows. One thread an orbit is
+// bound by its own instruction stream, 2240 cycles a step; here by the longest warp's, 1200. Wrapped standard map, MGS,
+// tau = 1, 10000 steps: 4099 orbits 11.4 -> 6.2 ms, 9472 orbits 11.2 -> 7.3; tau = 4 4.6 -> 3.2.
+template <class Sys, class Est>
+__global__ void __launch_bounds__(160, 2) record_pipe_kernel(const RecArgs a, const Sys sys) {
+    constexpr int S = Sys::S, D = Sys::D, K = 2, NCOL = K + 7 + S, B = PIPE_STEPS;
+    using M = Measure<D, K, double, Est>;
+    using P = PipeParts<Sys, Est, M, K, true>;
+    using EstState = typename Est::template State<D, K>;
+    constexpr int EW = sizeof(EstState) / 8, MW = sizeof(MonState) / 8;
+    extern __shared__ __align__(16) unsigned char record_smem[];
+    typename P::Shared& sh = *reinterpret_cast<typename P::Shared*>(record_smem);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const i64 orbit = static_cast<i64>(blockIdx.x) * 32 + lane;
+    const bool mine = orbit < a.n;
+    const i64 i = mine ? orbit : a.n - 1;       // spare lanes follow the last orbit and store nothing
+    const int H = a.tau < B ? B / a.tau : 1;    // handoffs a block
+    const i64 handoffs = a.steps / a.tau, blocks = (handoffs + H - 1) / H;
+    auto in_block = [&](i64 b) { return static_cast<int>(min(static_cast<i64>(H), handoffs - b * H)); };
+
+    const bool was = a.n0 == 0 || a.code[i] == STATUS_OK;
+    double x[S], W[D * K];
+    StdJac J;
+#pragma unroll
+    for (int c = 0; c < S; ++c) x[c] = a.x[i * S + c];
+#pragma unroll
+    for (int l = 0; l < D * K; ++l) W[l] = a.W[i * D * K + l];
+    Chain<D, K, Est> est;
+    MonState mon;
+    uint64_t* st = a.states + i * (EW + MW);
+    uint64_t* ew = reinterpret_cast<uint64_t*>(&est.head);
+    uint64_t* mw = reinterpret_cast<uint64_t*>(&mon);
+    i64 n = a.n0;
+    int8_t code = STATUS_OK;
+    bool alive = was;
+    int g = 0, ghi = -1;   // the next grid step and the last inside the launch
+    double* Ri = a.R + i * static_cast<i64>(NCOL) * a.n_grid;
+    i64 due = 0;           // its step count
+    auto rows = [&]() {    // the rows whose segment has no further handoff (record_kernel's loop over the grid)
+        while (due - n < a.tau) {
+            double lam[K], orth, gmax;
+            EstFinal<Est>::get(est.head, lam, orth, gmax);
+            if (mine) record_row<S, K>(Ri, g, lam, orth, gmax, mon, x);
+            due = ++g <= ghi ? a.grid[g] : INT64_MAX;
+        }
+    };
+    if (warp == 4) {
+#pragma unroll
+        for (int w = 0; w < EW; ++w) ew[w] = a.n0 == 0 ? 0ull : st[w];
+#pragma unroll
+        for (int w = 0; w < MW; ++w) mw[w] = a.n0 == 0 ? 0ull : st[EW + w];
+        while (g < a.n_grid && a.grid[g] <= a.n0) ++g;
+        ghi = g - 1;
+        while (ghi + 1 < a.n_grid && a.grid[ghi + 1] <= a.n0 + a.steps) ++ghi;
+        due = g <= ghi ? a.grid[g] : INT64_MAX;
+        if (alive) rows();
+    }
+    if (warp == 0) sys.jac(x, J);
+    if (threadIdx.x == 0) sh.running = 1;
+    __syncthreads();
+
+    for (i64 p = 0; p < blocks + 3; ++p) {
+        if (warp == 0) {
+            if (p < blocks) P::points(sh, sys, x, J, p, in_block(p), a.tau, lane);
+        } else if (warp == 1) {
+            const i64 b = p - 1;
+            if (b >= 0 && b < blocks) P::frames(sh, sys, W, a.prm.orthogonality_tol, b, in_block(b), a.tau, lane);
+        } else if (warp < 4) {
+            const i64 b = p - 2;
+            if (b >= 0 && b < blocks) P::measures(sh, &a.prm, b, in_block(b), warp - 2, lane);
+        } else {
+            const i64 b = p - 3;
+            if (b >= 0) {
+                const int hs = in_block(b);
+                for (int h = 0; h < hs; ++h) {
+                    if (!alive) break;
+                    M m;
+                    P::arrive(sh, W, x, m, b, h, lane);
+                    n += a.tau;
+                    code = all_finite_x<D, S>(x) ? (all_finite<D * K>(W) ? STATUS_OK : STATUS_W) : STATUS_STATE;
+                    if (code == STATUS_OK) {
+                        int pend = 0;
+                        est.template run<true, false>(n, W, &a.prm, m, pend);
+                        StdJac Jn;
+                        Jn.s = 0.0;
+                        Jn.c = sh.sj[b & 3][h][lane];
+                        monitor_ahead(sys, x, Jn, mon);
+                        if (est.failed()) code = STATUS_REDUCER;
+                        else if (n == a.N) code = all_finite<D * K>(W) ? STATUS_OK : STATUS_W;   // orbit.jl:58, x is finite here
+                    }
+                    if (code != STATUS_OK) {
+                        if (mine) a.fail[i] = g + 1;
+                        alive = false;
+                    } else {
+                        rows();
+                    }
+                }
+                const bool any = __any_sync(0xffffffffu, alive);
+                if (lane == 0) sh.running = any;
+            }
+        }
+        __syncthreads();
+        if (!sh.running) break;
+        __syncthreads();   // `running` is read before the next block may write it
+    }
+    if (warp != 4 || !mine || !was) return;
+#pragma unroll
+    for (int k2 = 0; k2 < S; ++k2) a.x[i * S + k2] = x[k2];
+#pragma unroll
+    for (int l = 0; l < D * K; ++l) a.W[i * D * K + l] = W[l];
+#pragma unroll
+    for (int w = 0; w < EW; ++w) st[w] = ew[w];
+#pragma unroll
+    for (int w = 0; w < MW; ++w) st[EW + w] = mw[w];
+    a.code[i] = code;
+    if (a.hstep) a.hstep[i] = n;
+}
+
 typedef cudaError_t (*RecordFn)(const cl_run& run, const RecArgs& a, cudaStream_t st);
 
 template <class Sys, class Est, int K, typename Real>
 cudaError_t launch_record(const cl_run& run, const RecArgs& a, cudaStream_t st) {
     const Sys sys = SysMaker<Sys>::make(run, nullptr);
+    // the orbit kernel's own line (cl_pipe.cuh): two blocks an SM, and handoffs often enough. At the line, 9472 orbits x
+    // 10000 steps, MGS / Householder: tau = 1 7.3 / 6.6 ms against 11.2 / 10.4 one thread an orbit, tau = 4 3.2 / 3.2
+    // against 4.6 / 4.4.
+    if constexpr (PipeOf<Sys, Real, Frame<K, Est>, 1>::ok && K == 2) {
+        if (a.tau <= PIPE_STEPS && a.n <= PIPE_ORBITS) {
+            auto k = record_pipe_kernel<Sys, Est>;
+            constexpr int smem = sizeof(typename PipeParts<Sys, Est, Measure<2, K, double, Est>, K, true>::Shared);
+            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (e != cudaSuccess) return e;
+            k<<<static_cast<unsigned>((a.n + 31) / 32), 160, smem, st>>>(a, sys);
+            return cudaGetLastError();
+        }
+    }
     record_kernel<Sys, Est, K, Real><<<static_cast<unsigned>((a.n + 127) / 128), 128, 0, st>>>(a, sys);
     return cudaGetLastError();
 }
