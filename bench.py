@@ -104,22 +104,28 @@ def flops_per_orbit_step(tau: int = TAU, precision: str = "fp64", n_steps: int =
 
 
 class ClockSampler:
-    """nvidia-smi samples of SM clock and throttle reasons during the timed region (200 ms period)."""
+    """nvidia-smi samples of SM clock and throttle reasons during the timed region (100 ms period). The region begins
+    once the tool has given its first sample (its start takes longer than the shorter regions), which is dropped;
+    wait=False for regions of microseconds, which an idle spell before them slows down."""
 
     Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,clocks_event_reasons.hw_slowdown,"
          "clocks_event_reasons.hw_thermal_slowdown,clocks_event_reasons.sw_thermal_slowdown,"
          "clocks_event_reasons.sw_power_cap")
 
-    def __init__(self, index: int):
-        self.index, self.proc, self.lines = index, None, []
+    def __init__(self, index: int, wait: bool = True):
+        self.index, self.wait, self.proc, self.lines = index, wait, None, []
 
     def __enter__(self):
         try:
             self.proc = subprocess.Popen(["nvidia-smi", f"--id={self.index}", f"--query-gpu={self.Q}",
-                                          "--format=csv,noheader,nounits", "-lms", "200"],
+                                          "--format=csv,noheader,nounits", "-lms", "100"],
                                          stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.t = threading.Thread(target=self._read, daemon=True)
             self.t.start()
+            end = time.monotonic() + 5.0
+            while self.wait and not self.lines and self.proc.poll() is None and time.monotonic() < end:
+                time.sleep(0.01)
+            self.lines.clear()
         except OSError:
             self.proc = None
         return self
@@ -748,7 +754,7 @@ def workload_mlp(args):
     bwd = sum(2 * B * a * b for a, b in zip(fin, fout)) + sum(2 * B * a * b for a, b in zip(fin[1:], fout[1:]))
     out = torch.empty((B, OUT_PAD), dtype=torch.float32, device=dev)
     net.packed()
-    sampler = ClockSampler(0)
+    sampler = ClockSampler(0, wait=False)
     l0 = L.cl_b200_launch_count()
     ms_fused = _event_times(torch, dev, stream, lambda: net.forward_fused(X, out=out), args.steps, args.warmup, flush,
                             sampler)
