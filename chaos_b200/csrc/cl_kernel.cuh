@@ -352,9 +352,10 @@ __global__ void __launch_bounds__(128, MINB) orbit_kernel(const KArgs a, const S
     i64 n = a.n0;
     const i64 handoffs = a.steps / a.tau;
     for (i64 h = 0; h < handoffs; ++h) {
-        k0.take(fr0.W);
-        k1.take(fr1.W);
-        k2.take(fr2.W);
+        // a stopped frame's W no longer holds unit columns: its last ones stay kept while the other frames run on
+        if (NF == 1 || fr0.alive) k0.take(fr0.W);
+        if (NF > 1 && fr1.alive) k1.take(fr1.W);
+        if (NF > 2 && fr2.alive) k2.take(fr2.W);
         for (int t = AHEAD ? 1 : 0; t < a.tau; ++t) {
             if (!AHEAD) sys.jac(x, J);
             advance();
