@@ -212,8 +212,10 @@ def propagate_frames(sys: System, x0, N: int, frames: list[FrameSpec], *, tau: i
         return chunk_size(free, d, kk, reducer_bytes=rbytes, s=s) if free else n
 
     # Asking the driver for the free memory takes 0.2 ms, and tens of milliseconds beside other processes' work; a run
-    # of less than PROBE_BYTES is tried whole, and asks only if its allocation fails.
-    unprobed = chunk is None and n * (bytes_per_orbit(d, kk, s) + rbytes) <= PROBE_BYTES
+    # of less than PROBE_BYTES is tried whole, and asks only if its allocation fails. Hooked runs ask: their buffers
+    # come from torch, whose failure is not retried.
+    unprobed = (chunk is None and launch_plan.BEFORE_LAUNCH is None
+                and n * (bytes_per_orbit(d, kk, s) + rbytes) <= PROBE_BYTES)
     csize = chunk if chunk is not None else (n if unprobed else probed_chunk())
     csize = min(csize, cap, n) if n else 1
     x = np.empty((n, s))
