@@ -258,8 +258,11 @@ cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     cudaMemPool_t pool;
-    if (device_pool(dev, &pool) == 1) return cudaMallocFromPoolAsync(p, bytes, pool, st);
-    return cudaMalloc(p, bytes);
+    e = device_pool(dev, &pool) == 1 ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMalloc(p, bytes);
+    // A failed allocation is returned here and nowhere else: left in the runtime, the thread's next launch check would
+    // report it, and a caller that retries with less memory would fail there.
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    return e;
 }
 
 void pool_free(void* p, cudaStream_t st) {
