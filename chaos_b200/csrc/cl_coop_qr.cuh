@@ -41,7 +41,7 @@ template <int D, typename Real>
 __device__ __forceinline__ void coop_divide(const Real* v, Real by, Real* out) {
     if constexpr (sizeof(Real) == 8) {
         Ok ok;
-        ok.positive<800>(by);
+        ok.divisor(by);
         const double y = rcp64(by);
         double q[D];
 #pragma unroll

@@ -20,7 +20,8 @@
 // one, the instructions. Whole kernels before and after: wrapped standard map, MGS, tau = 1, 4096 orbits x 4000 steps
 // 11.09 -> 4.35 ms (65536 x 1000: 3.70 -> 2.09 ms); standard map, MEGNO + FLI + SALI, 20001 x 1000 4.73 -> 1.41 ms;
 // Froeschle map, Householder | GALI + SALI, tau = 10, 65536 x 1000 6.60 -> 2.27 ms.
-// tests/test_gpu_fast64.py holds each to the operators on random operands and on the operands nearest a tie.
+// tests/test_gpu_fast64.py holds each to the operators on random operands and on the operands nearest a tie,
+// tests/test_gpu_fast64_limits.py over the whole range that `Ok` accepts.
 #pragma once
 
 #include "cl_math.cuh"
@@ -35,6 +36,12 @@ struct Ok {
     template <int E>
     __device__ __forceinline__ void positive(double b) {
         constexpr unsigned lo = static_cast<unsigned>(1023 - E) << 20, span = static_cast<unsigned>(2 * E) << 20;
+        ok = ok && static_cast<unsigned>(__double2hiint(b)) - lo < span;
+    }
+    // The divisor of `dividend`s: positive, exponent from -800 to 209, so that no accepted quotient is below 2^-1010. (A
+    // bound relative to each divisor, for divisors up to 2^700, cost the lattices' handoffs 2-4 % of the kernel.)
+    __device__ __forceinline__ void divisor(double b) {
+        constexpr unsigned lo = static_cast<unsigned>(1023 - 800) << 20, span = static_cast<unsigned>(800 + 210) << 20;
         ok = ok && static_cast<unsigned>(__double2hiint(b)) - lo < span;
     }
     // a dividend: zero, or large enough that the quotient's residual is exact
@@ -160,6 +167,8 @@ struct QRFast {
     bool ok;
 };
 
+// The quotients' dividends are not checked: one too small to be exact belongs to an entry of R^{-1} so small that b, which
+// holds the pivots' inverse squares (at least 2^-200) and is at most 2^700, is the same with any such value in its place.
 template <int K>
 __device__ __forceinline__ double window_Gw64(const double* R, const double* rin, Ok& ok) {
     double m = 0.0;
@@ -230,6 +239,7 @@ __device__ __forceinline__ void gs64(const double* W, double* Q, double* R, doub
         }
         double y;
         const double gamma = norm64r<D>(u, ok, y);
+        ok.positive<100>(gamma);   // as every pivot; the other two factorisations divide by at most twice one
         R[m + m * K] = gamma;
         rin[m] = y;
 #pragma unroll
@@ -423,6 +433,7 @@ __device__ __forceinline__ void pair64(const double* W, Pair64& m) {
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
         m.a[j] = norm64r<D>(W + j * D, ok, m.y[j]);
+        ok.divisor(m.a[j]);
         m.lg[j] = log64(m.a[j]);
 #pragma unroll
         for (int i = 0; i < D; ++i) ok.dividend(W[i + j * D]);

@@ -64,6 +64,7 @@ __device__ __forceinline__ void pipe_next(double* W, double tol) {
         for (int j = 0; j < 2; ++j) {
             double y;
             a[j] = norm64r<D>(W + j * D, ok, y);
+            ok.divisor(a[j]);
 #pragma unroll
             for (int i = 0; i < D; ++i) { ok.dividend(W[i + j * D]); V[i + j * D] = quo64(W[i + j * D], a[j], y); }
         }

@@ -139,6 +139,7 @@ struct RBenettin {
             Ok ok;
             double y;
             const double a = norm64r<D>(W, ok, y), lg = log64(a);
+            ok.divisor(a);
             double u[D];
 #pragma unroll
             for (int l = 0; l < D; ++l) { ok.dividend(W[l]); u[l] = quo64(W[l], a, y); }
@@ -279,6 +280,7 @@ struct RGALI {
 #pragma unroll
             for (int j = 0; j < K; ++j) {
                 a[j] = norm64r<D>(W + j * D, ok, y[j]);
+                ok.divisor(a[j]);
                 lg[j] = log64(a[j]);
 #pragma unroll
                 for (int i = 0; i < D; ++i) ok.dividend(W[i + j * D]);
