@@ -20,13 +20,17 @@ def _cs(name):
     return [(name + "_s", "<f8"), (name + "_c", "<f8")]
 
 
-def _words(field, *shape):
-    """The Float64 words that follow a state's field, as a view: `shape` numbers them row-major within the record."""
-    strides, step = [], 8
-    for k in reversed(shape):
-        strides.insert(0, step)
-        step *= k
-    return np.lib.stride_tricks.as_strided(field, (len(field), *shape), (field.strides[0], *strides))
+def _columns(n, *cols):
+    """Columns of length n side by side as an array (n, len(cols)) of its own; a column is an array or (array, array), the
+    sum of the two. Written column by column: numpy's copy of an (n, 2) view runs row by row (84 against 34 us
+    at 20001 orbits)."""
+    out = np.empty((n, len(cols)))
+    for j, c in enumerate(cols):
+        if isinstance(c, tuple):
+            np.add(*c, out=out[:, j])
+        else:
+            out[:, j] = c
+    return out
 
 
 def _tot(s, c):
@@ -199,8 +203,7 @@ class SALI(Reducer):
 
     def finals(self, st, d=None):
         n = st["n"].astype(np.int64, copy=False)
-        v = _words(st["s1_s"], 2, 2)   # (column, sum / comp)
-        s, c = v[:, :, 0], v[:, :, 1]
+        s, c = _columns(len(n), st["s1_s"], st["s2_s"]), _columns(len(n), st["s1_c"], st["s2_c"])
         L = np.where(n == 0, 0.0, -((s[:, 0] + s[:, 1]) + (c[:, 0] + c[:, 1])))
         return dict(n=n, sali=st["sali"].astype(np.float64, copy=False), L=L, sum=s, comp=c, floor=np.full(len(n), 4 * EPS))
 
@@ -316,19 +319,18 @@ class MEGNO(Reducer):
                     sum=pair("s", "s"), comp=pair("s", "c"), R1=tot("R1"), R2=tot("R2"), Q=tot("Q"), Q2=tot("Q2"))
 
     def finals(self, st, d=None):
-        # (column, s R1 R2 Q Q2, sum / comp): one pass for every total instead of one per field
         n, K = st["n"].astype(np.int64, copy=False), st["K"].astype(np.int64, copy=False)
-        v = _words(st["c1_s_s"], 2, 5, 2)
-        tot = v[..., 0] + v[..., 1]
-        tn, zero = n.astype(np.float64)[:, None], (K == 0)[:, None]
+        N, tn, zero = len(n), n.astype(np.float64), K == 0
+        tot = {nm: _columns(N, *((st[f"{col}_{nm}_s"], st[f"{col}_{nm}_c"]) for col in ("c1", "c2")))
+               for nm in ("R1", "R2", "Q", "Q2")}
         with np.errstate(invalid="ignore", divide="ignore"):
-            safe = np.where(K == 0, 1, K)
-            nk = np.where(K == 0, 0, n // safe).astype(np.float64)[:, None]
-            Y = np.where(zero, 0.0, 2 * tot[:, :, 1] / tn)
-            Ybar = np.where(zero, 0.0, tot[:, :, 3] / K.astype(np.float64)[:, None])
-            Ybar20 = np.where(zero, 0.0, nk * tot[:, :, 4] / (tn * tn * tn))
-        return dict(n=n, handoffs=K, Y=Y, Ybar=Ybar, Ybar20=Ybar20, sum=v[:, :, 0, 0], comp=v[:, :, 0, 1],
-                    R1=tot[:, :, 1], R2=tot[:, :, 2], Q=tot[:, :, 3], Q2=tot[:, :, 4])
+            nk = np.where(zero, 0, n // np.where(zero, 1, K)).astype(np.float64)
+            tK, t3 = K.astype(np.float64), tn * tn * tn
+            Y = _columns(N, *(np.where(zero, 0.0, 2 * tot["R1"][:, j] / tn) for j in range(2)))
+            Ybar = _columns(N, *(np.where(zero, 0.0, tot["Q"][:, j] / tK) for j in range(2)))
+            Ybar20 = _columns(N, *(np.where(zero, 0.0, nk * tot["Q2"][:, j] / t3) for j in range(2)))
+        return dict(n=n, handoffs=K, Y=Y, Ybar=Ybar, Ybar20=Ybar20, sum=_columns(N, st["c1_s_s"], st["c2_s_s"]),
+                    comp=_columns(N, st["c1_s_c"], st["c2_s_c"]), **tot)
 
     def error(self, st, orbit, backend):
         v = float(st["value"])
@@ -369,9 +371,9 @@ class FLI(Reducer):
                     stepB=int(st["stepB"]), colB=int(st["colB"]), step1=int(st["step1"]))
 
     def finals(self, st, d=None):
-        v = _words(st["s1_s"], 2, 2)   # (column, sum / comp)
         return dict(n=st["n"].astype(np.int64, copy=False), fli=st["fB"].astype(np.float64, copy=False), fli1=st["f1"].astype(np.float64, copy=False),
-                    sum=v[:, :, 0], comp=v[:, :, 1],
+                    sum=_columns(len(st["n"]), st["s1_s"], st["s2_s"]),
+                    comp=_columns(len(st["n"]), st["s1_c"], st["s2_c"]),
                     stepB=st["stepB"].astype(np.int64, copy=False), colB=st["colB"].astype(np.int64, copy=False),
                     step1=st["step1"].astype(np.int64, copy=False))
 
