@@ -322,14 +322,4 @@ cudaError_t launch_ensemble_any(const cl_run& run, const EArgs& a, int grid, con
     return launch_ensemble<Sys, Real, F, U>(run, a, grid, t, st, info);
 }
 
-// Lanes per orbit of the cooperative form of a run (the lattice's site count), or 1 when it has none.
-inline int coop_lanes(const cl_run& r) {
-    if (r.sys.kind != CL_SYS_CHAIN || r.n_frames != 1) return 1;
-    const cl_frame& f = r.frames[0];
-    if (f.n_reducers != 1 || f.reducers[0].kind != CL_RED_QR || f.reducers[0].alg != CL_QR_HOUSEHOLDER) return 1;
-    const int ns = r.d / 2;
-    if ((ns != 2 && ns != 4 && ns != 8) || f.k % ns != 0) return 1;
-    return ns;
-}
-
 }  // namespace cl

@@ -10,6 +10,7 @@
 // ever waits on another: the queue is a counter, not a barrier.
 #pragma once
 
+#include "cl_ensemble_rule.h"
 #include "cl_kernel.cuh"
 #include "cl_registry.cuh"
 
@@ -124,8 +125,6 @@ __global__ void __launch_bounds__(128, MINB) ensemble_kernel(const EArgs a, Sys 
         if (a.hstep) a.hstep[i] = fr.hstep;
     }
 }
-
-struct ETune { int block, minb, unroll, lanes; };   // lanes: per orbit (1 = one orbit per thread)
 
 typedef cudaError_t (*ELaunchFn)(const cl_run& run, const EArgs& a, int grid, const ETune& t, cudaStream_t st,
                                  LaunchInfo* info);

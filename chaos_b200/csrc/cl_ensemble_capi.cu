@@ -44,40 +44,14 @@ int sm_count() {
 
 std::string tune_key(const cl_run& r) { return run_key(r) + "t" + std::to_string(r.tau); }
 
-// An untuned class of 4 or 8 sites takes the cooperative kernel (one orbit per 4 or 8 lanes), whose longest orbit
-// finishes several times sooner: at 10000 orbits a class and lengths to 1e5 (ms, one orbit per thread / cooperative)
-// d = 16 Float64 807 / 146, mixed 390 / 69; d = 8 Float64 602 / 197, mixed 127 / 115; the four classes together 415 / 145
-// mixed and 1043 / 249 Float64. It also carries the larger load of 65536 orbits a class, lengths to 2e4 (d = 16 Float64
-// 301 / 179, mixed 93 / 74; d = 8 Float64 137 / 103), but for d = 8 in mixed precision (31 / 40), whose frame fits one
-// thread's registers: that one goes back to a thread per orbit when those fill a block of every SM.
-bool coop_by_default(const cl_ensemble_class& c) {
-    const int lanes = coop_lanes(c.run);
-    if (lanes < 4 || !c.buf.W0[0]) return false;
-    return lanes > 4 || c.run.precision == CL_PREC_FP64 || c.n_orbits <= 128 * static_cast<int64_t>(sm_count());
-}
-
 ETune variant_of(const cl_ensemble_class& c) {
-    ETune t{128, 2, 1, 1};
-    if (coop_by_default(c)) {
-        t.lanes = coop_lanes(c.run);
-        // the window unrolled at the compiled tau: mixed d = 16 80 -> 69 ms, Float64 146 -> 184
-        if (c.run.precision != CL_PREC_FP64) t.unroll = c.run.tau;
-        // one block an SM while the class is a few rounds of them: the longest orbits set its time, and the other classes
-        // find room beside it (two blocks of these kernels fill an SM's registers); more rounds need both blocks
-        // (10000 orbits a class 142 against 145 ms; 65536 a class 209 against 131)
-        if (c.n_orbits * t.lanes <= 8 * 128 * static_cast<int64_t>(sm_count())) t.minb = 1;
-    }
+    ETune t = untuned_variant(c, sm_count());
     {
         std::lock_guard<std::mutex> g(g_tune_mu);
         auto it = g_tuned.find(tune_key(c.run));
         if (it != g_tuned.end()) t = it->second;
     }
-    if (c.minb > 0) t.minb = c.minb;
-    if (c.unroll > 0) t.unroll = c.unroll;
-    if (c.lanes > 0) t.lanes = c.lanes;
-    if (t.unroll != 1 && t.unroll != c.run.tau) t.unroll = 1;
-    if (t.lanes > 1 && (t.lanes != coop_lanes(c.run) || !c.buf.W0[0])) t.lanes = 1;
-    return t;
+    return asked_variant(c, t);
 }
 
 int check_class(const cl_ensemble_class& c, ELaunchFn* fn) {
