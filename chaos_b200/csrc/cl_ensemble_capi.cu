@@ -44,8 +44,9 @@ int sm_count() {
 
 std::string tune_key(const cl_run& r) { return run_key(r) + "t" + std::to_string(r.tau); }
 
-ETune variant_of(const cl_ensemble_class& c) {
-    ETune t = untuned_variant(c, sm_count());
+// beside: other classes of the call run on the device at the same time
+ETune variant_of(const cl_ensemble_class& c, bool beside) {
+    ETune t = untuned_variant(c, sm_count(), beside);
     {
         std::lock_guard<std::mutex> g(g_tune_mu);
         auto it = g_tuned.find(tune_key(c.run));
@@ -148,7 +149,7 @@ int enqueue_classes(const cl_ensemble_class* cs, int nc, unsigned long long* cou
         fk.streams.push_back(ss[c]);
         fk.events.push_back(done[c]);
         cudaStreamWaitEvent(ss[c], fork, 0);
-        const ETune t = variant_of(cs[c]);
+        const ETune t = variant_of(cs[c], nc > 1);
         const int grid = sms * t.minb;
         e = fns[c](cs[c].run, eargs(cs[c], counters + c), grid, t, ss[c], info);
         capi_count_launch();
@@ -189,7 +190,7 @@ int enqueue_classes_in_order(const cl_ensemble_class* cs, int nc, unsigned long 
     }
     const int sms = sm_count();
     for (int c = 0; c < nc; ++c) {
-        const ETune t = variant_of(cs[c]);
+        const ETune t = variant_of(cs[c], false);
         const cudaError_t e = fns[c](cs[c].run, eargs(cs[c], heads + c), sms * t.minb, t, st, nullptr);
         capi_count_launch();
         if (e != cudaSuccess) return capi_map_cuda(e, "ensemble kernel launch");

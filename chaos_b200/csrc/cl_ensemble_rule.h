@@ -33,7 +33,7 @@ inline bool coop_by_default(const cl_ensemble_class& c, int sms) {
 }
 
 // The settings of a class nobody tuned, in the form that runs it: such a class may ask for the one-thread kernel (lanes = 1).
-inline ETune untuned_variant(const cl_ensemble_class& c, int sms) {
+inline ETune untuned_variant(const cl_ensemble_class& c, int sms, bool beside) {
     ETune t{128, 2, 1, 1};
     if (!coop_by_default(c, sms)) return t;
     const int lanes = coop_lanes(c.run);
@@ -45,10 +45,13 @@ inline ETune untuned_variant(const cl_ensemble_class& c, int sms) {
         if (c.run.precision != CL_PREC_FP64) t.unroll = c.run.tau;
     }
     // One block an SM while the class is a few rounds of them: the longest orbits set its time, and a second block beside
-    // theirs slows them; beside other classes these take the room (two blocks of these kernels fill an SM's registers;
-    // 10000 orbits a class 142 against 145 ms; 65536 a class 209 against 131). One orbit per thread likewise (18000 orbits
-    // to 2e4, ms at one / two blocks: mixed d = 8 25 / 32, d = 16 78 / 85, Float64 120 / 121, 169 / 250).
-    if (c.n_orbits * lanes <= 8 * 128 * static_cast<int64_t>(sms)) t.minb = 1;
+    // theirs slows them. Up to 8 rounds beside other classes, which take the room (two blocks of these kernels fill an
+    // SM's registers; 10000 orbits a class 142 against 145 ms; 65536 a class 209 against 131), and for one orbit per
+    // thread (18000 orbits to 2e4, ms at one / two blocks: mixed d = 8 25 / 32, d = 16 78 / 85, Float64 120 / 121, 169 /
+    // 250). A cooperative class alone up to 5 (d = 16, lengths to 1e5: 4.6 rounds mixed 71 / 79, Float64 147 / 174; 5.5 85 /
+    // 81, 176 / 176; 6.3 98 / 80, 202 / 177; lengths to 2e4: 3.0 14.5 / 16.7, 29.8 / 35.3; 3.8 18.1 / 16.8, 36.2 / 35.4;
+    // 6.3 29.6 / 18.1, 61.6 / 38.9).
+    if (c.n_orbits * lanes <= (coop && !beside ? 5 : 8) * 128 * static_cast<int64_t>(sms)) t.minb = 1;
     return t;
 }
 
