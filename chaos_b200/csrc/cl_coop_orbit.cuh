@@ -445,11 +445,18 @@ cudaError_t launch_coop_orbit(const cl_run& run, const KArgs& a, cudaStream_t st
 // The variant number of the cooperative form in a lattice instance's variant set (bit V_COOP - 1 of its mask).
 constexpr int V_COOP = 8;
 
-// Orbits up to which an untuned run takes the cooperative form. Measured at N = 2e4, tau = 10, k = 8 (ms, one-thread
-// / cooperative): d = 16 at 512 and 2048 orbits 1.6-3x faster cooperatively (Float64 MGS 232 / 116, Float64 GALI
-// 295 / 186, mixed Householder 120 / 41), at 8192 about even (Float64 Householder 329 / 304, Float64 GALI 303 / 401),
-// slower at 65536 orbits (Float64 Householder 127 / 213 at N = 2000), where one thread per orbit already fills the
-// GPU; d = 8 Float64 1.2-1.9x faster at 2048 and 8192 (GALI 135 / 71).
+// Orbits up to which an untuned run takes the cooperative form. At N = 2000, tau = 10, k = 8 (ms, one-thread /
+// cooperative):      4096 orbits     8192           16384          65536
+//   d = 16 Float64 Householder  27.8 / 6.7   27.4 / 13.3    27.0 / 26.0    125 / 93
+//          MGS                  18.7 / 5.5   18.6 / 11.2    19.6 / 22.4     92 / 78
+//          GALI                  9.2 / 2.2    9.8 / 4.4     12.2 / 8.6      40 / 30
+//          mixed Householder    12.0 / 2.7   12.1 / 5.3     12.1 / 10.1     27 / 37
+//   d = 10 Float64 Householder  15.7 / 4.8   15.7 / 9.5     15.7 / 18.8     48 / 67
+//          mixed Householder     5.3 / 2.4    5.3 / 4.8      5.3 / 9.2      12 / 33
+//   d = 8  Float64 Householder  12.2 / 4.3   12.2 / 5.0     12.2 / 9.9      30 / 35
+//          mixed Householder     2.8 / 2.3    2.9 / 2.6      3.1 / 5.1       7 / 14
+// So the line is on the safe side: it was drawn when the cooperative handoffs took two to three times as long, and up to
+// 8192 orbits the cooperative form is the faster one now at each of these d.
 constexpr i64 kCoopMaxOrbits = 4096;
 
 // A lattice instance of `propagate` with d >= 8: variant 1 is the one-thread kernel, variant V_COOP the cooperative

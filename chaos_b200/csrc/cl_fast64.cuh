@@ -17,9 +17,10 @@
 //   root        the estimate rsqrt.approx.ftz.f64 refined cubically, then one residual correction (Markstein 1990).
 // Dependent latencies on a B200 (cycles): `/` 114, sqrt 182, cl_log 399; rcp64 76, a further quotient 30, root64 77,
 // log64 297, and independent ones overlap. What bounds a handoff of a small ensemble is the chain of these; of a large
-// one, the instructions. Whole kernels before and after: wrapped standard map, MGS, tau = 1, 4096 orbits x 4000 steps
-// 11.09 -> 4.35 ms (65536 x 1000: 3.70 -> 2.09 ms); standard map, MEGNO + FLI + SALI, 20001 x 1000 4.73 -> 1.41 ms;
-// Froeschle map, Householder | GALI + SALI, tau = 10, 65536 x 1000 6.60 -> 2.27 ms.
+// one, the instructions. Whole kernels before and after, one orbit a thread: wrapped standard map, MGS, tau = 1, 65536
+// orbits x 1000 steps 3.70 -> 2.09 ms (4096 x 4000 11.09 -> 4.35, before the pipeline of cl_pipe.cuh took that size, now
+// 2.49); standard map, MEGNO + FLI + SALI, 20001 x 1000 4.73 -> 1.43 ms; Froeschle map, Householder | GALI + SALI, tau =
+// 10, 65536 x 1000 6.60 -> 2.29 ms.
 // tests/test_gpu_fast64.py holds each to the operators on random operands and on the operands nearest a tie,
 // tests/test_gpu_fast64_limits.py over the whole range that `Ok` accepts.
 #pragma once

@@ -13,9 +13,12 @@
 // runs; once warp 4 has stopped an orbit, what the others compute for it is not looked at. The warps work on blocks of
 // PIPE_STEPS steps, each one block behind the one before it, and meet at a barrier after each block.
 // Wrapped standard map, MGS, tau = 1, 4736 orbits x 1000 steps: 0.96 -> 0.63 ms; standard map, Householder, tau = 4 0.31 ->
-// 0.21, MEGNO + FLI + SALI 1.21 -> 0.99 (there warp 4's sums are the longest). The line is two blocks an SM, which its
-// registers hold: 9472 orbits 0.96 -> 0.70 ms, 14208 orbits 0.97 against 1.41 the other way. Above tau = PIPE_STEPS the
-// handoffs are too few for the split to pay.
+// 0.21, MEGNO + FLI + SALI 1.21 -> 0.97 (there warp 4's sums are the longest). The line is two blocks an SM, which its
+// registers hold: 9472 orbits 0.96 -> 0.70 ms, 14208 orbits 0.97 against 1.41 the other way. Every chain gains at the line
+// (standard map, 9472 x 1000, one orbit a thread / pipeline, tau = 1 | tau = 4): MGS .94/.70 | .33/.26, CGS .94/.70 |
+// .32/.25, Householder .91/.64 | .32/.25, Givens .75/.50 | .28/.20, SALI .85/.57 | .30/.22, MEGNO 1.00/.73 | .34/.27, FLI
+// .81/.59 | .29/.22, MEGNO + SALI 1.11/.90 | .37/.31, FLI + SALI .95/.69 | .33/.25, MEGNO + FLI + SALI 1.22/1.05 | .40/.38.
+// Above tau = PIPE_STEPS the handoffs are too few for the split to pay.
 #pragma once
 
 #include <type_traits>

@@ -130,8 +130,8 @@ struct SysStandard {
 
 // _reduce (wrapped_standard_map.jl:15-28): a = floor(u / tp) from the IEEE quotient, three operations by the rounded
 // reciprocal of the constant (cl_fast64.cuh) and no branch: the step's point chain and the handoff's stay in one block
-// of straight-line code (wrapped standard map, MGS, tau = 1, 4096 x 4000: 4.36 -> 3.84 ms against the branch to a
-// division near integers). A non-finite u gives a NaN quotient and remainder, and the guards below see it. The
+// of straight-line code (wrapped standard map, MGS, tau = 1, 4096 x 4000, one orbit a thread as that size then ran: 4.36 ->
+// 3.84 ms against the branch to a division near integers). A non-finite u gives a NaN quotient and remainder, and the guards below see it. The
 // remainder and the guards are the reference's.
 __device__ __forceinline__ void wrap_reduce(double u, double tp, double& r, double& a) {
     a = floor(quo64(u, tp, 1.0 / tp));

@@ -375,7 +375,9 @@ def propagate(sys: System, x0, N: int, *, k: int, tau: int = 1, seed: int = 0, r
               finals: bool = True) -> PropagationResult:
     """propagate(sys, x0, N; k, tau=1, seed, reducers=(), backend=:gpu, chunk=nothing, W0=nothing) on the B200
     (src/Tangent/propagate.jl:267-290). `x0` is (n, s); `W0` (n, d, k) or None for the seeded frames;
-    `precision` is "fp64" (the reference's arithmetic) or "mixed" (Float32 tangent frames)."""
+    `precision` is "fp64" (the reference's arithmetic) or "mixed" (Float32 tangent frames). "mixed" is not always the
+    faster one: small ensembles of the two-dimensional maps (at most 9472 orbits at tau <= 4) and the splitting step
+    (KahanLi(8), 16384 orbits) run faster in "fp64"."""
     if backend not in ("gpu", "auto"):
         raise ValueError("backend must be :gpu or :auto here; the CPU path is the reference's own")
     return propagate_frames(sys, x0, N, [FrameSpec(int(k), tuple(reducers), W0)], tau=tau, seed=seed,
