@@ -49,6 +49,11 @@ class RecordResult:
         return self.R[:, :, k + COLUMNS.index(name) - 1]
 
 
+def _columns_of(W0) -> np.ndarray:
+    """The frames (n, d, k) with the columns of d contiguous, in an array of their own: the run leaves its frames there."""
+    return np.array(np.asarray(W0).transpose(0, 2, 1), dtype=np.float64, order="C")
+
+
 def record(sys, x0, N: int, tau: int, estimator, grid, *, W0=None, launch_steps: int | None = None,
            precision: str = "fp64") -> RecordResult:
     """Record n orbits of `sys` (StandardMap, WrappedStandardMap or a 2 x 2 LinearSymplecticMap) with `estimator`
@@ -76,7 +81,7 @@ def record(sys, x0, N: int, tau: int, estimator, grid, *, W0=None, launch_steps:
     sb = Lb.cl_b200_record_state_bytes(C.byref(run))
     if W0 is None:
         W0 = np.broadcast_to(np.eye(d)[:, :k], (n, d, k))
-    Wc = np.ascontiguousarray(np.asarray(W0, dtype=np.float64).transpose(0, 2, 1))   # columns of d contiguous
+    Wc = _columns_of(W0)
     x = x0.copy()
     states = np.zeros((n, sb), np.uint8)
     code = np.zeros(n, np.int8)
@@ -193,7 +198,7 @@ def record_indicators(sys, x0, N: int, tau: int, members, grid, *, ns: int = 2, 
     sb = Lb.cl_b200_indicator_state_bytes(C.byref(run))
     if W0 is None:
         W0 = np.broadcast_to(np.eye(d)[:, :2], (n, d, 2))
-    Wc = np.ascontiguousarray(np.asarray(W0, dtype=np.float64).transpose(0, 2, 1))
+    Wc = _columns_of(W0)
     x = x0.copy()
     states = np.zeros((n, sb), np.uint8)
     code = np.zeros(n, np.int8)
@@ -313,7 +318,7 @@ def record_indicator_pairs(sys, z0, W0, N: int, tau: int, members, grid, *, ns: 
     if ncol < 0:
         raise ValueError(f"pair chain {members} is outside the compiled menu")
     sb = Lb.cl_b200_indicator_state_bytes(C.byref(run))
-    Wc = np.ascontiguousarray(W0.transpose(0, 2, 1))
+    Wc = _columns_of(W0)
     x = z0.copy()
     states = np.zeros((n, sb), np.uint8)
     code = np.zeros(n, np.int8)
